@@ -157,6 +157,7 @@ def _cairo(case, g):
 def prepare(case, seed):
     kind = case["kind"]
     g = _gen(seed)
+    api.init_memory_pool()  # once per device, as a program that uses the library does at start-up
     if kind == "commit":
         cols = _m31(g, case["n_cols"], 1 << case["log_n"])
         s = {"cols": cols, "lde": _empty(case["n_cols"], 1 << (case["log_n"] + case["blowup"])), "root": _empty(8)}
