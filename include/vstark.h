@@ -262,8 +262,9 @@ int vs_autotune_lde(uint32_t log_n, uint32_t n_cols, uint32_t blowup_bits, uint3
                     float* ms, uint32_t cap, vs_stream_t stream);
 /* Merkle subtree shape of the root-only trees (no counterpart in the reference):
  * the first reduction level stops at 2^split roots per 1024-leaf tile (0..8), so a
- * CTA skips the narrow top levels of its tile, and the next level reduces them.
- * Roots are identical for every split. Process wide; applies to vs_commit_columns,
+ * CTA skips the narrow top levels of its tile, and the next level reduces them; 0,
+ * the default, leaves the choice to the library, and trees below 2^20 leaves take
+ * smaller tiles of their own. Roots are identical for every split. Process wide; applies to vs_commit_columns,
  * vs_merkle_root_rowpacked / _capped / _soa4, vs_fri_fold_commit, the Cairo FRI and
  * the engine's commitment jobs (their scratch is sized for split 8). */
 int vs_merkle_split_set(uint32_t split);

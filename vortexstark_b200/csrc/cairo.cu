@@ -926,7 +926,7 @@ extern "C" int vs_cairo_oods_fri(void* channel, vs_cairo_oods_fri_io* io, vs_str
   uint32_t *fri = nullptr, *mscratch = nullptr;
   VS_TRY(s.alloc(&fri, 4 * N));
   VS_TRY(s.alloc(&mscratch, merkle_scratch_words_any(N / 2)));
-  const uint32_t split = merkle_split();
+  const uint32_t split = std::min<uint32_t>(merkle_root_split(log_eval), 5);
   uint32_t* src[4] = {oq[0], oq[1], oq[2], oq[3]};
   uint32_t* dst[4];
   uint64_t off = 0;

@@ -314,7 +314,7 @@ struct Engine {
     const uint64_t n = 1ull << j.log_n, N = n << 2;
     VS_TRY(vs_fill_uniform_m31(c.cols, (uint64_t)j.n_cols * n, j.seed, 0, (vs_stream_t)st));
     VS_TRY(lde_cached(TW_STWO, c.cols, n, c.lde, N, j.n_cols, j.log_n, 2, st));
-    VS_TRY(merkle_root(LeafRowPacked{c.lde, N, j.n_cols}, N, c.root, st, c.scratch, merkle_split()));
+    VS_TRY(merkle_root(LeafRowPacked{c.lde, N, j.n_cols}, N, c.root, st, c.scratch, merkle_root_split(j.log_n + 2)));
     VS_CUDA(cudaMemcpyAsync(c.h_root, c.root, 32, cudaMemcpyDeviceToHost, st));
     VS_CUDA(cudaStreamSynchronize(st));
     outs[0].assign((uint8_t*)c.h_root, (uint8_t*)c.h_root + 32);

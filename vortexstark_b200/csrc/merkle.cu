@@ -147,20 +147,20 @@ int vs_merkle_root_rowpacked(const uint32_t* d_cols, uint64_t stride, uint32_t n
   clear_error();
   if (!d_cols || !d_root || log_leaves > 31) return set_error(VS_ERR_INVALID, "vs_merkle_root_rowpacked: bad args");
   return merkle_root(LeafRowPacked{d_cols, stride, n_cols}, 1ull << log_leaves, d_root, (cudaStream_t)st, nullptr,
-                     merkle_split());
+                     merkle_root_split(log_leaves));
 }
 int vs_merkle_root_capped(const uint32_t* d_cols, uint64_t stride, uint32_t n_cols, uint32_t log_leaves,
                           uint32_t* d_root, vs_stream_t st) {
   clear_error();
   if (!d_cols || !d_root || log_leaves > 31) return set_error(VS_ERR_INVALID, "vs_merkle_root_capped: bad args");
   return merkle_root(LeafCapped{nullptr, d_cols, stride, n_cols}, 1ull << log_leaves, d_root, (cudaStream_t)st, nullptr,
-                     merkle_split());
+                     merkle_root_split(log_leaves));
 }
 int vs_merkle_root_soa4(const uint32_t* c0, const uint32_t* c1, const uint32_t* c2, const uint32_t* c3,
                         uint32_t log_leaves, uint32_t* d_root, vs_stream_t st) {
   clear_error();
   if (!c0 || !c1 || !c2 || !c3 || !d_root || log_leaves > 31) return set_error(VS_ERR_INVALID, "vs_merkle_root_soa4: bad args");
-  return merkle_root(LeafSoa4{c0, c1, c2, c3}, 1ull << log_leaves, d_root, (cudaStream_t)st, nullptr, merkle_split());
+  return merkle_root(LeafSoa4{c0, c1, c2, c3}, 1ull << log_leaves, d_root, (cudaStream_t)st, nullptr, merkle_root_split(log_leaves));
 }
 
 int vs_merkle_split_set(uint32_t split) {

@@ -26,32 +26,53 @@ int merkle_tile_roots(const Leaf& leaf, uint64_t n_leaves, uint32_t TL, uint32_t
   return VS_OK;
 }
 
-// Largest split merkle_root accepts: the first level may stop at 2^8 roots per
-// 1024-leaf tile (the level where all 256 threads of a CTA still have a node).
+// Largest split a caller may set (vs_merkle_split_set): 2^8 roots left per 1024-leaf
+// tile, the level where all 256 threads of a CTA still have a node.
 constexpr uint32_t MK_MAX_SPLIT = 8;
-// Process-wide split of the root-only trees (vs_merkle_split_set).
+// Process-wide split (vs_merkle_split_set); 0 leaves the choice to merkle_root_split.
 uint32_t merkle_split();
 
-// Split of a reduction level over `cur` hashes: the leaf level takes the split
-// as given; hash levels of at least 2^20 hashes (1024+ CTAs) take at most 5 (each
-// step then reduces 32-fold, so the chain stays short), smaller ones reduce each
-// tile to one root.
-inline uint32_t merkle_level_split(uint64_t cur, uint32_t split) {
-  return cur >= (1ull << 20) ? std::min<uint32_t>(split, 5) : 0u;
+// From 2^MK_WIDE leaves on, the rate of compressions bounds a root-only tree: its
+// 1024-leaf tiles stop at 2^split roots, where a level still fills warps, and the next
+// level takes them over. Below, the chain of dependent compressions does (log2(n)
+// levels): tiles are smaller, so that every SM has some and a thread hashes one or two
+// leaves in a row and not four.
+constexpr uint32_t MK_WIDE = 20;
+// Split of a wide tree of 2^L leaves when none is set: 7, the fastest (row-packed root
+// of 34 x 2^26: 11.90 / 11.64 / 11.30 / 11.42 ms at 5 / 6 / 7 / 8), less where its
+// roots would take more than 256 MB of scratch.
+inline uint32_t merkle_root_split(uint32_t L) {
+  const uint32_t s = merkle_split();
+  return s ? s : (L <= 26 ? 7u : 33u - L);
+}
+// Tile of a reduction level over 2^L leaves, or over 2^L hashes of the level before:
+// 2^TL of them, reduced to 2^stop. Measured on whole roots (us, one 1024-leaf tile a CTA
+// and one root a tile, then this rule; 34 / 16 columns): 2^12 leaves 43 -> 23 / 31 -> 23,
+// 2^16 46 -> 33 / 36 -> 29, 2^18 74 -> 68 / 51 -> 47, 2^19 132 -> 109 / 84 -> 70.
+// Split 0, for callers with little scratch, leaves one root a tile from 2^18 on.
+struct MerkleTile {
+  uint32_t TL, stop;
+};
+inline MerkleTile merkle_tile(uint32_t L, bool hashes, uint32_t split) {
+  if (L <= (hashes ? 10u : 8u)) return {L, 0};
+  if (L <= 14) return {7, 0};
+  if (L <= 17) return {L - 7, 0};
+  if (L < MK_WIDE) return split ? MerkleTile{L - 10, 7} : MerkleTile{MK_MAX_TL, 0};
+  return {MK_MAX_TL, split};
 }
 
 // Words of scratch merkle_root needs for n_leaves leaves with split `split` (0 when
-// n_leaves <= 1024): the sum of the hash levels it writes, in the order it writes
-// them (merkle_root follows the same sequence).
+// one CTA does): the sum of the hash levels it writes, in the order it writes them
+// (merkle_root follows the same sequence).
 inline uint64_t merkle_scratch_words(uint64_t n_leaves, uint32_t split = 0) {
-  if (n_leaves <= (1ull << MK_MAX_TL)) return 0;
-  uint64_t cur = n_leaves >> (MK_MAX_TL - split);
-  uint64_t words = cur * 8;
-  while (cur > (1ull << MK_MAX_TL)) {
-    cur >>= MK_MAX_TL - merkle_level_split(cur, split);
-    words += cur * 8;
+  uint64_t words = 0;
+  uint32_t L = ilog2(n_leaves);
+  for (bool hashes = false;; hashes = true) {
+    const MerkleTile t = merkle_tile(L, hashes, split);
+    if (t.TL == L && !t.stop) return words;
+    L -= t.TL - t.stop;
+    words += 8ull << L;
   }
-  return words;
 }
 // Split used for trees that keep their 1024-leaf tile roots (prover trees of
 // 2^20+ leaves): tiles stop at 2^split subtree roots and `split` node launches
@@ -83,31 +104,33 @@ inline uint64_t merkle_scratch_words_any(uint64_t n_leaves) {
 // Root of a power-of-two tree whose leaves come from `leaf`. Intermediate tile
 // roots go to `scratch` (merkle_scratch_words(n_leaves, split) words; when null it
 // is allocated stream-ordered for the call). Each reduction level is written after
-// the previous one, never in place. The first level stops at 2^split roots per
-// 1024-leaf tile (split <= MK_MAX_SPLIT); the root is the same for every split.
+// the previous one, never in place. Levels of 2^MK_WIDE and more stop at 2^split roots
+// per 1024-leaf tile (split <= MK_MAX_SPLIT); the root is the same for every split.
 template <class Leaf>
 int merkle_root(const Leaf& leaf, uint64_t n_leaves, uint32_t* d_root, cudaStream_t st, uint32_t* scratch = nullptr,
                 uint32_t split = 0) {
   if (!is_pow2(n_leaves)) return set_error(VS_ERR_INVALID, "merkle: leaf count %llu is not a power of two",
                                            (unsigned long long)n_leaves);
   if (split > MK_MAX_SPLIT) return set_error(VS_ERR_INVALID, "merkle: split %u above %u", split, MK_MAX_SPLIT);
-  const uint32_t L = ilog2(n_leaves);
-  if (L <= MK_MAX_TL) return merkle_tile_roots(leaf, n_leaves, L, d_root, st);
-  uint32_t* buf = scratch;
-  if (!buf) VS_CUDA(cudaMallocAsync((void**)&buf, merkle_scratch_words(n_leaves, split) * 4, st));
-  uint64_t cur = n_leaves >> (MK_MAX_TL - split);
-  int rc = merkle_tile_roots(leaf, n_leaves, MK_MAX_TL, buf, st, split);
-  uint32_t* level = buf;
-  while (rc == VS_OK) {
-    const uint32_t Lc = ilog2(cur);
-    if (Lc <= MK_MAX_TL) { rc = merkle_tile_roots(LeafHashes{level}, cur, Lc, d_root, st); break; }
-    uint32_t* next = level + cur * 8;
-    const uint32_t sp = merkle_level_split(cur, split);
-    rc = merkle_tile_roots(LeafHashes{level}, cur, MK_MAX_TL, next, st, sp);
-    level = next;
-    cur >>= MK_MAX_TL - sp;
+  const uint64_t words = merkle_scratch_words(n_leaves, split);
+  uint32_t *level = scratch, *buf = nullptr;
+  if (words && !scratch) {
+    VS_CUDA(cudaMallocAsync((void**)&buf, words * 4, st));
+    level = buf;
   }
-  if (!scratch) {
+  uint32_t L = ilog2(n_leaves);
+  MerkleTile t = merkle_tile(L, false, split);
+  bool last = t.TL == L && !t.stop;
+  int rc = merkle_tile_roots(leaf, n_leaves, t.TL, last ? d_root : level, st, t.stop);
+  while (rc == VS_OK && !last) {
+    L -= t.TL - t.stop;
+    t = merkle_tile(L, true, split);
+    last = t.TL == L && !t.stop;
+    uint32_t* next = level + (8ull << L);
+    rc = merkle_tile_roots(LeafHashes{level}, 1ull << L, t.TL, last ? d_root : next, st, t.stop);
+    level = next;
+  }
+  if (buf) {
     cudaError_t e = cudaFreeAsync(buf, st);
     if (rc == VS_OK) rc = check_cuda(e, "merkle scratch free");
   }

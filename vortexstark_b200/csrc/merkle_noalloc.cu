@@ -19,7 +19,7 @@ namespace vs {
 // Largest tree this entry point accepts, and the scratch that tree needs: one
 // 8-word subtree root per 1024 leaves plus the next reduction level.
 constexpr uint32_t NOALLOC_MAX_LOG_LEAVES = 26;
-constexpr uint64_t NOALLOC_SCRATCH_WORDS = ((1ull << (NOALLOC_MAX_LOG_LEAVES - 10)) + 64) * 8;  // 2.1 MB
+constexpr uint64_t NOALLOC_SCRATCH_WORDS = ((1ull << (NOALLOC_MAX_LOG_LEAVES - 10)) + 128) * 8;  // 2.1 MB
 
 // Every GPU that loads the library holds this array until the process exits.
 // All calls on a device share it and it keeps the last call's contents; calls
@@ -104,10 +104,12 @@ extern "C" int vs_merkle_root_rowpacked_noalloc(const uint32_t* d_cols, uint64_t
                      log_leaves, NOALLOC_MAX_LOG_LEAVES);
   const uint64_t n = 1ull << log_leaves;
   uint32_t* scratch = nullptr;  // trees of at most 1024 leaves need no scratch
-  if (merkle_scratch_words(n) > NOALLOC_SCRATCH_WORDS)
+  uint32_t split = merkle_root_split(log_leaves);  // as wide a first level as the array holds
+  while (split && merkle_scratch_words(n, split) > NOALLOC_SCRATCH_WORDS) split--;
+  if (merkle_scratch_words(n, split) > NOALLOC_SCRATCH_WORDS)
     return set_error(VS_ERR_INVALID, "vs_merkle_root_rowpacked_noalloc: scratch for 2^%u leaves exceeds the array",
                      log_leaves);
-  if (merkle_scratch_words(n) > 0) VS_TRY(noalloc_scratch(&scratch));
+  if (merkle_scratch_words(n, split) > 0) VS_TRY(noalloc_scratch(&scratch));
   // With scratch supplied (or not needed) merkle_root performs no allocation.
-  return merkle_root(LeafRowPacked{d_cols, stride, n_cols}, n, d_root, (cudaStream_t)st, scratch);
+  return merkle_root(LeafRowPacked{d_cols, stride, n_cols}, n, d_root, (cudaStream_t)st, scratch, split);
 }
