@@ -61,6 +61,22 @@ inline MerkleTile merkle_tile(uint32_t L, bool hashes, uint32_t split) {
   return {MK_MAX_TL, split};
 }
 
+// A forest's CTAs for tiles of at most 2^TL leaves; trees are added largest first.
+inline void merkle_forest_add(MerkleForest& f, uint32_t TL, uint32_t log_n, const uint32_t* src, uint32_t* out) {
+  f.log_n[f.n] = log_n;
+  f.src[f.n] = src;
+  f.out[f.n] = out;
+  f.start[f.n + 1] = f.start[f.n] + (1u << (log_n - std::min(TL, log_n)));
+  f.n++;
+}
+template <class Leaf>
+int merkle_forest(const MerkleForest& f, uint32_t TL, cudaStream_t st) {
+  if (!f.n) return VS_OK;
+  merkle_forest_kernel<Leaf><<<f.start[f.n], MK_THREADS, merkle_smem_bytes(TL), st>>>(f, TL);
+  VS_LAUNCHED("merkle_forest_kernel");
+  return VS_OK;
+}
+
 // Words of scratch merkle_root needs for n_leaves leaves with split `split` (0 when
 // one CTA does): the sum of the hash levels it writes, in the order it writes them
 // (merkle_root follows the same sequence).
