@@ -1,0 +1,34 @@
+"""vs_prove_fib at the trace sizes between those of test_gpu_prover.py (trees that end in one
+launch or two, layers inside and above the last-layers kernel), and from several threads on
+streams of their own, byte for byte against the oracle."""
+import threading
+
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+torch = pytest.importorskip("torch")
+import oracle_lib as O  # noqa: E402
+from vortexstark_b200 import api  # noqa: E402
+
+
+@pytest.mark.parametrize("log_n", [4, 7, 9, 13, 15, 17, 18])
+def test_proof_bytes(log_n):
+    assert api.prove_fib(3, 1000 + log_n, log_n) == O.prove(3, 1000 + log_n, log_n)
+
+
+def test_threads_and_streams():
+    sizes = (6, 9, 12, 14)
+    exp = {k: O.prove(1, 7 + k, k) for k in sizes}
+    got = {}
+
+    def work(k):
+        st = torch.cuda.Stream()
+        got[k] = [api.prove_fib(1, 7 + k, k, stream=st) for _ in range(4)]
+
+    th = [threading.Thread(target=work, args=(k,)) for k in sizes]
+    for t in th:
+        t.start()
+    for t in th:
+        t.join()
+    assert all(got[k] == [exp[k]] * 4 for k in sizes)

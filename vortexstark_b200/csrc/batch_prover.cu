@@ -17,10 +17,10 @@
 //     draw, whose squeezes are independent given the state);
 //   * decommitment: one warp per (job, query) gathers its authentication path.
 //
-// Trees keep every level from level 3 up (eight-leaf groups): an authentication
-// path is a gather of the stored siblings plus the recomputation of one
-// eight-leaf group, instead of one 1024-leaf tile per query and tree as in the
-// tile-root provers (the reference keeps whole trees at these sizes too,
+// Trees keep every level from level 3 up (eight-leaf groups; 6 in the trees of single
+// proofs above 2^22 leaves): an authentication path is a gather of the stored
+// siblings plus the recomputation of one group, instead of one 1024-leaf tile per
+// query and tree as in the tile-root provers (the reference keeps whole trees at these sizes too,
 // MerkleTree::commit, src/prover.rs:1764-1766). The arithmetic, transcript and
 // proof layout are the graph prover's: every proof is byte-identical to
 // vs_prove_fib's for the same (a, b, log_n).
@@ -38,6 +38,7 @@
 #include "ntt.h"
 #include "prover.h"
 #include "prover_graph.h"
+#include "transcript_tree.cuh"
 #include "twiddles.h"
 #include "vs_common.cuh"
 
@@ -45,9 +46,12 @@ namespace vs {
 
 namespace {
 
-constexpr int BMAXF = 24;        // FRI layers for log_eval <= 27 (log_n <= BATCH_MAX_LOG_N + 3)
-constexpr uint32_t BGROUP = 3;   // lowest stored tree level: 2^3-leaf groups are recomputed
-constexpr uint32_t BTOP = 10;    // tree_top_kernel takes the last levels of <= 2^10 hashes per tree
+constexpr int BMAXF = 28;  // FRI layers for log_eval <= 30
+// Lowest kept level of a tree of 2^m leaves: an opened leaf's group of 2^s is hashed again.
+// Eight-leaf groups cost 8 bytes a leaf; trees above 2^22 leaves keep 64-leaf groups (1
+// byte a leaf), which one warp still hashes at once.
+constexpr uint32_t BGROUP_MAX = 6;
+constexpr uint32_t group_log(uint32_t m) { return m > 22 ? BGROUP_MAX : (m < 3 ? m : 3); }
 
 // ------------------------------------------------------------------ batched leaf functors
 // Global leaf g of a batch of trees with 2^log_len leaves each: job g >> log_len,
@@ -119,158 +123,74 @@ struct LeafFoldB {
   }
 };
 
-// Stored levels of a batch of trees with 2^m leaves each: lv[k - s] is level k
-// (k = s..m), [jobs][2^(m-k)] hashes of 8 words.
-struct TreeLevels {
-  uint32_t* lv[32];
-  uint32_t s, m;
-};
-
 // ------------------------------------------------------------------ kernels
-// One CTA per tree: levels k0+1..m from level k0 (2^(m-k0) <= 2^BTOP hashes per
-// tree), each written to its stored level. Shared memory: two hash buffers.
-__global__ void __launch_bounds__(256) tree_top_kernel(TreeLevels t, uint32_t k0) {
-  extern __shared__ uint32_t tt_sm[];
-  const uint32_t j = blockIdx.x;
-  uint32_t cnt = 1u << (t.m - k0);
-  uint32_t* a = tt_sm;
-  uint32_t* b = tt_sm + 8 * cnt;
-  const uint32_t* src = t.lv[k0 - t.s] + (uint64_t)j * cnt * 8;
-  for (uint32_t i = threadIdx.x; i < 8 * cnt; i += blockDim.x) a[i] = src[i];
-  __syncthreads();
-  for (uint32_t k = k0 + 1; k <= t.m; k++) {
-    cnt >>= 1;
-    uint32_t* dst = t.lv[k - t.s] + (uint64_t)j * cnt * 8;
-    for (uint32_t i = threadIdx.x; i < cnt; i += blockDim.x) {
-      uint32_t h[8];
-      b2s_node(h, a + 16 * i, a + 16 * i + 8);
-#pragma unroll
-      for (int w = 0; w < 8; w++) { b[8 * i + w] = h[w]; dst[8 * i + w] = h[w]; }
-    }
-    __syncthreads();
-    uint32_t* tmp = a;
-    a = b;
-    b = tmp;
-  }
-}
-
-// Channel of job j (one thread each): mix a root (copied into the job's arena)
-// and, when alpha_off >= 0, draw a challenge into the job's alpha slots.
-__global__ void bch_mix_draw_kernel(ChanDev* ch, uint32_t jobs, int reset, const uint32_t* __restrict__ roots,
-                                    uint32_t* arena, uint64_t words, uint64_t arena_off, uint32_t* alpha,
-                                    uint32_t astride, int alpha_off) {
-  const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
-  if (j >= jobs) return;
-  ChanDev c = ch[j];
-  if (reset) {
-    for (int i = 0; i < 8; i++) c.state[i] = 0;
-    c.n_draws = 0;
-    c.error = 0;
-  }
-  uint32_t r[8];
-  uint32_t* ar = arena + (uint64_t)j * words + arena_off;
-  for (int i = 0; i < 8; i++) { r[i] = roots[8 * j + i]; ar[i] = r[i]; }
-  ch_mix_digest(c, r);
-  if (alpha_off >= 0) {
-    uint32_t v[4];
-    ch_draw_felt(c, v);
-    for (int i = 0; i < 4; i++) alpha[(uint64_t)j * astride + alpha_off + i] = v[i];
-  }
-  ch[j] = c;
-}
-
-// One CTA per job: mix_felts(last layer), then the N_QUERIES draw_number squeezes,
-// which depend only on the state and their draw counter, in parallel.
-__global__ void __launch_bounds__(96) bch_queries_kernel(ChanDev* ch, const uint32_t* l0, const uint32_t* l1,
-                                                        const uint32_t* l2, const uint32_t* l3, uint32_t* arena,
-                                                        uint64_t words, uint64_t a_last, uint64_t a_q,
-                                                        uint32_t* qidx, uint32_t log_eval) {
-  __shared__ ChanDev sc;
-  const uint32_t j = blockIdx.x;
-  uint32_t* ar = arena + (uint64_t)j * words;
-  if (threadIdx.x == 0) {
-    ChanDev c = ch[j];
-    const uint32_t* planes[4] = {l0 + 8 * j, l1 + 8 * j, l2 + 8 * j, l3 + 8 * j};
-    for (int i = 0; i < 8; i++)
-      for (int k = 0; k < 4; k++) ar[a_last + 4 * i + k] = planes[k][i];
-    ch_mix_felts_planes(c, planes, 8);
-    sc = c;
-  }
-  __syncthreads();
-  if (threadIdx.x < N_QUERIES) {
-    ChanDev c = sc;
-    c.n_draws = threadIdx.x;  // the q-th draw after the mix squeezes with counter q
-    const uint32_t v = ch_draw_pow2(c, log_eval);
-    qidx[j * N_QUERIES + threadIdx.x] = v;
-    ar[a_q + threadIdx.x] = v;
-  }
-  if (threadIdx.x == 0) {
-    ChanDev c = sc;
-    c.n_draws = N_QUERIES;
-    ch[j] = c;
-  }
-}
-
-struct BDecParams {
+// Decommitment of every tree in one launch: blockIdx.y is the tree (trace, quotient, FRI
+// layers), a warp takes one (job, query): the opened values and the authentication paths
+// of leaf f (the query, or q >> (l+1) in FRI layer l) and of its sibling f ^ 1. Levels
+// below s come from recomputing f's 2^s-leaf group, levels s..m-1 from the kept ones.
+struct BDecommit {
   const uint32_t* eval;
-  uint32_t log_eval;
+  uint32_t log_eval, nf, jobs;
   const uint32_t* alpha;
   uint32_t astride;
   const uint32_t* qidx;
   uint32_t* arena;
-  uint64_t words, a_tv, a_qv, a_fv;
-  uint32_t nf;
+  uint64_t words, a_tv, a_qv, a_fv[BMAXF], a_tree[2 + BMAXF];
   const uint32_t* fri[BMAXF][4];  // plane k of layer l: [jobs][2^(log_eval-1-l)]
+  TreeLevels tree[2 + BMAXF];
 };
-// One CTA per job: values at each query and its fold sibling (q ^ 1); FRI layer l
-// uses q >> (l + 1).
-__global__ void bdecommit_values_kernel(BDecParams p) {
-  const uint32_t t = threadIdx.x, j = blockIdx.x;
-  if (t >= 2 * N_QUERIES) return;
-  const uint32_t qi = t % N_QUERIES, sib = t >= N_QUERIES ? 1u : 0u;
-  const uint32_t q = p.qidx[j * N_QUERIES + qi];
-  const uint32_t i = q ^ sib;
-  const uint32_t mask = (1u << p.log_eval) - 1;
-  const uint32_t* e = p.eval + ((uint64_t)j << p.log_eval);
-  uint32_t* ar = p.arena + (uint64_t)j * p.words;
-  ar[p.a_tv + t] = e[i];
-  const uint32_t* al = p.alpha + (uint64_t)j * p.astride;
-  const qm31 a{{al[0], al[1], al[2], al[3]}};
-  const qm31 qv = qscale(a, sub(e[(i + 2) & mask], add(e[(i + 1) & mask], e[i])));
-  for (int k = 0; k < 4; k++) ar[p.a_qv + 4 * t + k] = qv.v[k];
-  for (uint32_t l = 0; l < p.nf; l++) {
-    const uint32_t f = (q >> (l + 1)) ^ sib;
-    const uint64_t base = (uint64_t)j << (p.log_eval - 1 - l);
-    for (int k = 0; k < 4; k++) ar[p.a_fv + (l * 2 * N_QUERIES + t) * 4 + k] = p.fri[l][k][base + f];
-  }
-}
-
-// One warp per (job, query): the authentication paths of leaf f = qidx >> shift and
-// of its sibling f ^ 1. Levels below s come from recomputing f's 2^s-leaf group
-// (side-effect-free leaf functor), levels s..m-1 from the stored levels.
-template <class Leaf>
-__global__ void __launch_bounds__(256) bpaths_kernel(Leaf leaf, TreeLevels t, uint32_t shift,
-                                                    const uint32_t* __restrict__ qidx, uint32_t jobs,
-                                                    uint32_t* __restrict__ arena, uint64_t words, uint64_t off) {
-  __shared__ uint32_t sm[8][(2 << BGROUP) * 8];
-  const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+__global__ void __launch_bounds__(256) batch_decommit_kernel(BDecommit p) {
+  __shared__ __align__(16) uint32_t sm[8][(2 << BGROUP_MAX) * 8];
+  const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31, y = blockIdx.y;
   const uint32_t wi = blockIdx.x * 8 + warp;
-  if (wi >= jobs * N_QUERIES) return;  // uniform per warp
+  if (wi >= p.jobs * N_QUERIES) return;  // uniform per warp
   const uint32_t j = wi / N_QUERIES, qi = wi % N_QUERIES;
+  const TreeLevels t = p.tree[y];
   const uint32_t s = t.s, m = t.m, g = 1u << s;
-  const uint32_t f = qidx[j * N_QUERIES + qi] >> shift;
-  uint32_t* S = sm[warp];
-  const uint64_t gbase = ((uint64_t)j << m) + ((uint64_t)(f >> s) << s);
-  if (lane < g) {
-    uint32_t h[8];
-    leaf(gbase + lane, h);
+  const uint32_t f = p.qidx[j * N_QUERIES + qi] >> (y < 2 ? 0 : y - 1);
+  const uint32_t* al = p.alpha + (uint64_t)j * p.astride;
+  // the words of leaf i of this job's tree
+  auto words = [&](uint32_t i, uint32_t w[4]) {
+    if (y == 0) {
+      w[0] = p.eval[((uint64_t)j << m) + i];
+      w[1] = w[2] = w[3] = 0;
+    } else if (y == 1) {
+      const uint32_t* e = p.eval + ((uint64_t)j << m);
+      const uint32_t mask = (1u << m) - 1;
+      const qm31 q = qscale(qm31{{al[0], al[1], al[2], al[3]}}, sub(e[(i + 2) & mask], add(e[(i + 1) & mask], e[i])));
 #pragma unroll
-    for (int w = 0; w < 8; w++) S[8 * lane + w] = h[w];
+      for (int k = 0; k < 4; k++) w[k] = q.v[k];
+    } else {
+#pragma unroll
+      for (int k = 0; k < 4; k++) w[k] = p.fri[y - 2][k][((uint64_t)j << m) + i];
+    }
+  };
+  uint32_t* ar = p.arena + (uint64_t)j * p.words;
+  uint32_t* S = sm[warp];
+  for (uint32_t x = lane; x < g; x += 32) {
+    const uint32_t i = ((f >> s) << s) + x;
+    uint32_t w[4], h[8], msg[16] = {0};
+    words(i, w);
+    if ((i ^ f) <= 1) {  // the query's leaf or its sibling: an opened value
+      const uint32_t at = ((i ^ f) & 1 ? N_QUERIES : 0) + qi;
+      if (y == 0) {
+        ar[p.a_tv + at] = w[0];
+      } else {
+        uint32_t* o = ar + (y == 1 ? p.a_qv : p.a_fv[y - 2]) + 4 * at;
+#pragma unroll
+        for (int k = 0; k < 4; k++) o[k] = w[k];
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < 4; k++) msg[k] = w[k];
+    b2s_single(h, msg, y == 0 ? 1 : 4);
+#pragma unroll
+    for (int k = 0; k < 8; k++) S[8 * x + k] = h[k];
   }
   __syncwarp();
   uint32_t lo = 0, cnt = g;
   for (uint32_t k = 1; k < s; k++) {
-    if (lane < cnt / 2) {
+    if (lane < cnt / 2) {  // at most 32 nodes
       uint32_t h[8];
       b2s_node(h, S + 8 * (lo + 2 * lane), S + 8 * (lo + 2 * lane + 1));
 #pragma unroll
@@ -280,21 +200,16 @@ __global__ void __launch_bounds__(256) bpaths_kernel(Leaf leaf, TreeLevels t, ui
     lo += cnt;
     cnt >>= 1;
   }
-  uint32_t* out = arena + (uint64_t)j * words + off;
-  for (uint32_t x = lane; x < 2 * m; x += 32) {
-    const uint32_t sd = x / m, k = x % m;
-    const uint32_t leaf_idx = f ^ sd;
-    uint32_t* dst = out + ((uint64_t)(sd * N_QUERIES + qi) * m + k) * 8;
+  uint32_t* out = ar + p.a_tree[y];
+  // a lane copies one word: eight lanes a hash
+  for (uint32_t x = lane >> 3; x < 2 * m; x += 4) {
+    const uint32_t sd = x / m, k = x % m, i = f ^ sd;
     const uint32_t* src;
-    if (k < s) {
-      uint32_t l0 = 0, lc = g;
-      for (uint32_t z = 0; z < k; z++) { l0 += lc; lc >>= 1; }
-      src = S + 8 * (l0 + (((leaf_idx & (g - 1)) >> k) ^ 1));
-    } else {
-      src = t.lv[k - s] + (((uint64_t)j << (m - k)) + ((leaf_idx >> k) ^ 1)) * 8;
-    }
-#pragma unroll
-    for (int w = 0; w < 8; w++) dst[w] = src[w];
+    if (k < s) src = S + 8 * (2 * g - (2 * g >> k) + (((i & (g - 1)) >> k) ^ 1));
+    else src = t.level(k) + (((uint64_t)j << (m - k)) + ((i >> k) ^ 1)) * 8;
+    uint32_t* path = out + (uint64_t)(sd * N_QUERIES + qi) * (1 + 8 * m);
+    if (k == 0 && (lane & 7) == 0) path[0] = m;
+    path[1 + 8 * k + (lane & 7)] = src[lane & 7];
   }
 }
 
@@ -314,10 +229,7 @@ struct BatchProver::Impl {
   uint32_t *d_ab = nullptr, *d_trace = nullptr, *d_eval = nullptr, *d_alpha = nullptr, *d_qidx = nullptr,
            *d_arena = nullptr;
   ChanDev* d_ch = nullptr;
-  struct Tree {
-    TreeLevels L{};
-    uint32_t TL = 0;
-  } trace_t, quot_t, fri_t[BMAXF];
+  TreeLevels trace_t{}, quot_t{}, fri_t[BMAXF] = {};
   uint32_t* fri[BMAXF][4] = {};
   ArenaLayout lay;
   std::map<uint32_t, cudaGraphExec_t> exec;  // per batch size
@@ -352,11 +264,9 @@ struct BatchProver::Impl {
       const uint64_t half = N >> (l + 1);
       for (int k = 0; k < 4; k++) fri[l][k] = (uint32_t*)take(4 * half * cap);
     }
-    auto tree = [&](Tree& t, uint32_t m) {
-      t.L.m = m;
-      t.L.s = std::min(BGROUP, m);
-      t.TL = std::min<uint32_t>(MK_MAX_TL, m);
-      for (uint32_t k = t.L.s; k <= m; k++) t.L.lv[k - t.L.s] = (uint32_t*)take(32ull * cap << (m - k));
+    auto tree = [&](TreeLevels& t, uint32_t m) {
+      t = TreeLevels{nullptr, cap, group_log(m), m};
+      t.base = (uint32_t*)take(TreeLevels::bytes(cap, t.s, m));
     };
     tree(trace_t, log_eval);
     tree(quot_t, log_eval);
@@ -376,69 +286,52 @@ struct BatchProver::Impl {
     total = carve(nullptr);
   }
 
-  template <class Leaf>
-  int commit(const Leaf& leaf, Tree& t, uint32_t b) {
-    const uint32_t s = t.L.s, m = t.L.m;
-    VS_TRY(merkle_tile_roots(leaf, (uint64_t)b << m, t.TL, t.L.lv[0], st, t.TL - s));
-    uint32_t k = s;
-    for (; m - k > BTOP; k++)
-      VS_TRY(launch_hash_nodes(t.L.lv[k - s], t.L.lv[k + 1 - s], (uint64_t)b << (m - k - 1), st));
-    if (k < m) {
-      const unsigned smem = (unsigned)(((1u << (m - k)) * 3 / 2) * 32);
-      tree_top_kernel<<<b, 256, smem, st>>>(t.L, k);
-      VS_LAUNCHED("tree_top_kernel");
-    }
-    return VS_OK;
+  ChannelStep step(int reset, uint64_t arena_off, int alpha_off) const {
+    return {d_ch, reset, d_arena, lay.words, arena_off, d_alpha, astride, alpha_off};
   }
-  template <class Leaf>
-  int paths(const Leaf& leaf, const Tree& t, uint32_t shift, size_t arena_off, uint32_t b) {
-    bpaths_kernel<Leaf><<<blocks_for((uint64_t)b * N_QUERIES, 8), 256, 0, st>>>(leaf, t.L, shift, d_qidx, b, d_arena,
-                                                                                 lay.words, arena_off);
-    VS_LAUNCHED("bpaths_kernel");
-    return VS_OK;
-  }
-
-  // The whole batch of b proofs, stream-ordered on st.
+  // The whole batch of b proofs, stream-ordered on st, from the public inputs in h_ab
+  // to the arenas in h_arena.
   int enqueue(uint32_t b) {
     VS_CUDA(cudaMemcpyAsync(d_ab, h_ab, 8ull * b, cudaMemcpyHostToDevice, st));
     fib_trace_params_kernel<<<dim3(blocks_for(n, 256 * 32), b), 256, 0, st>>>(d_ab, d_trace, n);
     VS_LAUNCHED("fib_trace_params_kernel");
     VS_TRY(lde_cached(TW_NATIVE, d_trace, n, d_eval, N, b, log_n, BLOWUP_BITS, st));
-    const unsigned cb = blocks_for(b, 64);
-    VS_TRY(commit(LeafOne{d_eval}, trace_t, b));
-    bch_mix_draw_kernel<<<cb, 64, 0, st>>>(d_ch, b, 1, trace_t.L.lv[trace_t.L.m - trace_t.L.s], d_arena, lay.words,
-                                           lay.roots, d_alpha, astride, 0);
-    VS_LAUNCHED("bch_mix_draw_kernel");
+    VS_TRY(commit_with_channel(LeafOne{d_eval}, trace_t, b, step(1, lay.root(0), 0), st));
     const LeafFibQuotB quot{d_eval, log_eval, d_alpha, astride};
-    VS_TRY(commit(quot, quot_t, b));
-    bch_mix_draw_kernel<<<cb, 64, 0, st>>>(d_ch, b, 0, quot_t.L.lv[quot_t.L.m - quot_t.L.s], d_arena, lay.words,
-                                           lay.roots + 8, d_alpha, astride, 4);
-    VS_LAUNCHED("bch_mix_draw_kernel");
+    VS_TRY(commit_with_channel(quot, quot_t, b, step(0, lay.root(1), 4), st));
+    FriTail tail{};
     for (uint32_t l = 0; l < nf; l++) {
       const uint32_t cur = log_eval - l;
       const uint32_t* tw = nullptr;
       VS_TRY(get_fold_twiddles(l == 0 ? COSET_HALF_COSET : COSET_HALF_ODDS, cur, &tw, st));
+      const ChannelStep c = step(0, lay.root(2 + l), l + 1 < nf ? (int)(4 * (2 + l)) : -1);
       if (l == 0) {
         LeafFoldQuotB leaf{quot, tw, cur - 1, d_alpha + 4, astride, {fri[0][0], fri[0][1], fri[0][2], fri[0][3]}};
-        VS_TRY(commit(leaf, fri_t[0], b));
-      } else {
+        VS_TRY(commit_with_channel(leaf, fri_t[0], b, c, st));
+      } else if (cur - 1 > TAIL_LOG) {
         LeafFoldB leaf{{fri[l - 1][0], fri[l - 1][1], fri[l - 1][2], fri[l - 1][3]},
                        {fri[l][0], fri[l][1], fri[l][2], fri[l][3]}, tw, cur - 1, d_alpha + 4 * (1 + l), astride};
-        VS_TRY(commit(leaf, fri_t[l], b));
+        VS_TRY(commit_with_channel(leaf, fri_t[l], b, c, st));
+      } else if (!tail.first) {
+        tail.first = l;
+        tail.step = c;
       }
-      const Tree& t = fri_t[l];
-      bch_mix_draw_kernel<<<cb, 64, 0, st>>>(d_ch, b, 0, t.L.lv[t.L.m - t.L.s], d_arena, lay.words,
-                                             lay.roots + 8 * (2 + l), d_alpha, astride,
-                                             l + 1 < nf ? (int)(4 * (2 + l)) : -1);
-      VS_LAUNCHED("bch_mix_draw_kernel");
+      tail.tw[l] = tw;
+      tail.tree[l] = fri_t[l];
+      for (int k = 0; k < 4; k++) tail.fri[l][k] = fri[l][k];
     }
-    const auto& last = fri[nf - 1];
-    bch_queries_kernel<<<b, 96, 0, st>>>(d_ch, last[0], last[1], last[2], last[3], d_arena, lay.words, lay.last,
-                                         lay.q, d_qidx, log_eval);
-    VS_LAUNCHED("bch_queries_kernel");
-    BDecParams dp{};
+    tail.nf = nf;
+    tail.log_eval = log_eval;
+    tail.a_last = lay.last;
+    tail.a_q = lay.q;
+    tail.qidx = d_qidx;
+    tail.alpha0 = 4;
+    VS_TRY(launch_fri_tail<true>(tail, b, st));
+    BDecommit dp{};
     dp.eval = d_eval;
     dp.log_eval = log_eval;
+    dp.nf = nf;
+    dp.jobs = b;
     dp.alpha = d_alpha;
     dp.astride = astride;
     dp.qidx = d_qidx;
@@ -446,16 +339,16 @@ struct BatchProver::Impl {
     dp.words = lay.words;
     dp.a_tv = lay.tv;
     dp.a_qv = lay.qv;
-    dp.a_fv = lay.fv;
-    dp.nf = nf;
-    for (uint32_t l = 0; l < nf; l++)
+    dp.tree[0] = trace_t;
+    dp.tree[1] = quot_t;
+    for (uint32_t y = 0; y < 2 + nf; y++) dp.a_tree[y] = lay.tree[y];
+    for (uint32_t l = 0; l < nf; l++) {
+      dp.tree[2 + l] = fri_t[l];
+      dp.a_fv[l] = lay.fv[l];
       for (int k = 0; k < 4; k++) dp.fri[l][k] = fri[l][k];
-    bdecommit_values_kernel<<<b, 2 * N_QUERIES, 0, st>>>(dp);
-    VS_LAUNCHED("bdecommit_values_kernel");
-    VS_TRY(paths(LeafOne{d_eval}, trace_t, 0, lay.tree[0], b));
-    VS_TRY(paths(quot, quot_t, 0, lay.tree[1], b));
-    for (uint32_t l = 0; l < nf; l++)
-      VS_TRY(paths(LeafSoa4{fri[l][0], fri[l][1], fri[l][2], fri[l][3]}, fri_t[l], l + 1, lay.tree[2 + l], b));
+    }
+    batch_decommit_kernel<<<dim3(blocks_for((uint64_t)b * N_QUERIES, 8), 2 + nf), 256, 0, st>>>(dp);
+    VS_LAUNCHED("batch_decommit_kernel");
     VS_CUDA(cudaMemcpyAsync(h_arena, d_arena, 4ull * lay.words * b, cudaMemcpyDeviceToHost, st));
     return VS_OK;
   }
@@ -522,6 +415,34 @@ struct BatchProver::Impl {
   }
 };
 
+int BatchProver::prove_once(uint32_t a, uint32_t b, uint32_t log_n, uint8_t* out, uint64_t cap, uint64_t* out_len,
+                            cudaStream_t st) {
+  Impl p;
+  p.plan(log_n, 1);
+  if (out_len) *out_len = p.lay.bytes();
+  if (!out || cap < p.lay.bytes())
+    return set_error(VS_ERR_INVALID, "proof needs %llu bytes, buffer has %llu", (unsigned long long)p.lay.bytes(),
+                     (unsigned long long)cap);
+  uint8_t* mem = nullptr;
+  cudaError_t e = cudaMallocAsync((void**)&mem, p.total, st);
+  if (e != cudaSuccess)
+    return set_error(VS_ERR_OOM, "proof workspace (%llu bytes): %s", (unsigned long long)p.total, cudaGetErrorString(e));
+  p.carve(mem);
+  uint32_t ab[2] = {a, b};
+  p.st = st;
+  p.h_ab = ab;
+  p.h_arena = reinterpret_cast<uint32_t*>(out);  // only the copy's destination
+  int rc = p.enqueue(1);
+  p.st = nullptr;  // the caller's stream and buffer are not the workspace's to release
+  p.h_ab = p.h_arena = nullptr;
+  cudaFreeAsync(mem, st);
+  e = cudaStreamSynchronize(st);
+  VS_TRY(rc);
+  VS_CUDA(e);
+  p.lay.finish(out, a, b);
+  return VS_OK;
+}
+
 BatchProver::BatchProver() : impl(new Impl) {}
 BatchProver::~BatchProver() = default;
 
@@ -563,16 +484,21 @@ int BatchProver::finish(std::vector<std::vector<uint8_t>>& out) {
   impl->running = nullptr;  // the launch stream may be reused for other work from here on
   const uint32_t count = impl->count;
   out.resize(count);
-  auto ser = [&](uint32_t j0, uint32_t step) {
-    for (uint32_t j = j0; j < count; j += step)
-      impl->lay.serialize(impl->h_arena + (uint64_t)j * impl->lay.words, impl->h_ab[2 * j], impl->h_ab[2 * j + 1],
-                          out[j]);
+  for (uint32_t j = 0; j < count; j++) {
+    uint8_t* proof = reinterpret_cast<uint8_t*>(impl->h_arena + (uint64_t)j * impl->lay.words);
+    impl->lay.finish(proof, impl->h_ab[2 * j], impl->h_ab[2 * j + 1]);
+  }
+  // copied out on up to 8 host threads
+  auto take = [&](uint32_t j0, uint32_t step) {
+    for (uint32_t j = j0; j < count; j += step) {
+      const uint8_t* proof = reinterpret_cast<const uint8_t*>(impl->h_arena + (uint64_t)j * impl->lay.words);
+      out[j].assign(proof, proof + impl->lay.bytes());
+    }
   };
-  // a batch's proofs are serialised on up to 8 host threads (about 0.1 ms per MB each)
   const uint32_t nt = std::min<uint32_t>(8, count / 4);
   std::vector<std::thread> th;
-  for (uint32_t t = 1; t < nt; t++) th.emplace_back(ser, t, nt);
-  ser(0, std::max<uint32_t>(nt, 1));
+  for (uint32_t t = 1; t < nt; t++) th.emplace_back(take, t, nt);
+  take(0, std::max<uint32_t>(nt, 1));
   for (auto& x : th) x.join();
   return VS_OK;
 }

@@ -30,6 +30,10 @@ class BatchProver {
   // (one batch in flight per instance); finish() waits and serialises each proof.
   int launch(const uint32_t* ab, uint32_t count, cudaStream_t on);
   int finish(std::vector<std::vector<uint8_t>>& out);
+  // One proof on `st`, as a batch of one without a workspace kept (stream-ordered
+  // allocation), written to the host buffer `out` when cap suffices; synchronises st.
+  static int prove_once(uint32_t a, uint32_t b, uint32_t log_n, uint8_t* out, uint64_t cap, uint64_t* out_len,
+                        cudaStream_t st);
   uint32_t log_n() const;
   uint32_t capacity() const;
   uint64_t device_bytes() const;

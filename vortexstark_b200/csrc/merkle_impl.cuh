@@ -25,13 +25,43 @@ constexpr int MK_MAX_TL = 10;
 // Shared memory: leaf layer (8 * 2^TL words) + next layer (8 * 2^(TL-1) words).
 inline unsigned merkle_smem_bytes(uint32_t TL) { return (8u << TL) * 4u + (TL ? (8u << (TL - 1)) * 4u : 0u); }
 
+// The kept levels of `jobs` equal trees of 2^m leaves each: level k (s <= k <= m) is
+// [jobs][2^(m-k)] hashes of 8 words, one level after the other.
+struct TreeLevels {
+  uint32_t* base;
+  uint32_t jobs, s, m;
+  __host__ __device__ uint32_t* level(uint32_t k) const {
+    return base + 8ull * jobs * ((2ull << (m - s)) - (2ull << (m - k)));
+  }
+  static uint64_t bytes(uint64_t jobs, uint32_t s, uint32_t m) { return 32ull * jobs * ((2ull << (m - s)) - 1); }
+};
+// Keeps a tile's levels: the tile's leaves are level k of the trees, it is tile `at` of
+// them, and a level of `half` hashes in the tile is level k + TL - log2(half).
+struct KeepLevels {
+  TreeLevels t;
+  uint64_t at;
+  uint32_t top;  // k + TL
+  __device__ __forceinline__ void operator()(uint32_t half, uint32_t i, const uint32_t h[8]) const {
+    const uint32_t k = top - (31 - __clz(half));
+    if (k < t.s) return;
+    uint4* g = reinterpret_cast<uint4*>(t.level(k)) + 2 * (at * half + i);
+    g[0] = make_uint4(h[0], h[1], h[2], h[3]);
+    g[1] = make_uint4(h[4], h[5], h[6], h[7]);
+  }
+};
+
+struct KeepNone {
+  __device__ __forceinline__ void operator()(uint32_t, uint32_t, const uint32_t*) const {}
+};
+
 // One tile: hashes 2^TL leaves from `base` and reduces them until n_out hashes are left in
 // shared memory, word w of hash j at the returned buffer's w * n_out + j.
+// Every level above the leaves goes to keep(half, i, hash) too.
 // MK_THREADS threads. (Kernels that hash their own way wrap this same code: written out
 // in another form, a level took 0.98 us in a lone CTA instead of 0.82.)
-template <class Leaf>
+template <class Leaf, class Keep>
 __device__ __forceinline__ uint32_t* merkle_tile_reduce(const Leaf& leaf, uint32_t TL, uint64_t base, uint64_t n_leaves,
-                                                        uint32_t n_out, uint32_t* mk_sm) {
+                                                        uint32_t n_out, uint32_t* mk_sm, const Keep& keep) {
   const uint32_t tile = 1u << TL;
   uint32_t* bufA = mk_sm;
   uint32_t* bufB = mk_sm + 8 * tile;
@@ -64,6 +94,7 @@ __device__ __forceinline__ uint32_t* merkle_tile_reduce(const Leaf& leaf, uint32
       b2s_compress(h, m, 64u, true);
 #pragma unroll
       for (int w = 0; w < 8; w++) nxt[w * half + i] = h[w];
+      keep(half, i, h);
     }
     __syncthreads();
     uint32_t* t = cur;
@@ -83,7 +114,7 @@ __global__ void __launch_bounds__(MK_THREADS) merkle_subtree_kernel(Leaf leaf, u
                                                                    uint32_t* __restrict__ roots, uint32_t stop_log) {
   extern __shared__ uint32_t mk_sm[];
   const uint32_t n_out = 1u << stop_log;
-  const uint32_t* cur = merkle_tile_reduce(leaf, TL, (uint64_t)blockIdx.x << TL, n_leaves, n_out, mk_sm);
+  const uint32_t* cur = merkle_tile_reduce(leaf, TL, (uint64_t)blockIdx.x << TL, n_leaves, n_out, mk_sm, KeepNone{});
   for (uint32_t i = threadIdx.x; i < 8 * n_out; i += MK_THREADS)
     roots[((uint64_t)blockIdx.x * n_out + (i >> 3)) * 8 + (i & 7)] = cur[(i & 7) * n_out + (i >> 3)];
 }
@@ -108,7 +139,7 @@ __global__ void __launch_bounds__(MK_THREADS) merkle_forest_kernel(MerkleForest 
   while (t + 1 < f.n && blockIdx.x >= f.start[t + 1]) t++;
   const uint32_t log_n = f.log_n[t], tl = min(TL, log_n), i0 = blockIdx.x - f.start[t];
   const uint64_t n = 1ull << log_n;
-  const uint32_t* cur = merkle_tile_reduce(Leaf::of(f.src[t], n), tl, (uint64_t)i0 << tl, n, 1, mk_sm);
+  const uint32_t* cur = merkle_tile_reduce(Leaf::of(f.src[t], n), tl, (uint64_t)i0 << tl, n, 1, mk_sm, KeepNone{});
   if (threadIdx.x < 8) f.out[t][8 * (uint64_t)i0 + threadIdx.x] = cur[threadIdx.x];
 }
 

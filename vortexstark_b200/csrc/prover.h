@@ -33,8 +33,6 @@ struct FibProof {
   std::vector<Decommit4> fri;
 };
 
-int prove_fib(uint32_t a, uint32_t b, uint32_t log_n, FibProof& pf, cudaStream_t st);
-std::vector<uint8_t> serialize(const FibProof& p);
 bool deserialize(const uint8_t* data, size_t len, FibProof& p);
 std::string verify(const FibProof& p);  // "" when accepted
 

@@ -1,6 +1,6 @@
 // Device-resident Fibonacci prover captured as one CUDA graph per trace size.
 //
-// Same arithmetic and transcript as prove_fib (prover.cu), restructured so no
+// Same arithmetic and transcript as the batched prover (batch_prover.cu): no
 // stage needs the host: the Fiat-Shamir channel runs on the device (one thread,
 // channel_dev.cuh), fold challenges are read by the fused leaf functors from
 // device memory, query indices are drawn on the device, and decommitment
@@ -160,7 +160,7 @@ struct DecParams {
   uint32_t* quot_vals;   // 2 x 80 x 4
   uint32_t nf;
   const uint32_t* fri[MAXF][4];
-  uint32_t* fri_vals;    // nf x 2 x 80 x 4
+  uint32_t* fri_vals[MAXF];  // 2 x 80 x 4 per layer
 };
 // Values at each query and its fold sibling (q ^ 1); FRI layer l uses q >> (l+1).
 __global__ void decommit_values_kernel(DecParams p) {
@@ -174,7 +174,7 @@ __global__ void decommit_values_kernel(DecParams p) {
   for (int k = 0; k < 4; k++) p.quot_vals[4 * t + k] = q.v[k];
   for (uint32_t l = 0; l < p.nf; l++) {
     const uint32_t f = (p.qidx[qi] >> (l + 1)) ^ (t >= N_QUERIES ? 1u : 0u);
-    for (int k = 0; k < 4; k++) p.fri_vals[(l * 2 * N_QUERIES + t) * 4 + k] = p.fri[l][k][f];
+    for (int k = 0; k < 4; k++) p.fri_vals[l][4 * t + k] = p.fri[l][k][f];
   }
 }
 
@@ -213,7 +213,9 @@ __global__ void __launch_bounds__(256) paths_kernel(Leaf leaf, uint32_t TL, uint
   for (uint32_t t = threadIdx.x; t < 2 * depth; t += blockDim.x) {
     const uint32_t s = t / depth, k = t % depth;
     const uint32_t leaf_idx = f ^ s;
-    uint32_t* dst = out + ((uint64_t)(s * N_QUERIES + qi) * depth + k) * 8;
+    uint32_t* path = out + (uint64_t)(s * N_QUERIES + qi) * (1 + 8 * depth);
+    uint32_t* dst = path + 1 + 8 * k;
+    if (k == 0) path[0] = depth;
     if (k < TL) {
       uint32_t lo = 0, lc = n0;
       for (uint32_t j = 0; j < k; j++) { lo += lc; lc >>= 1; }
@@ -232,60 +234,42 @@ void ArenaLayout::plan(uint32_t ln) {
   log_n = ln;
   log_eval = ln + BLOWUP_BITS;
   nf = log_eval - LOG_LAST_LAYER;
+  fv.clear();
   tree.clear();
   depth.clear();
-  size_t w = 0;
-  roots = w; w += 8 * (2 + nf);
-  last = w; w += 32;
-  q = w; w += N_QUERIES;
+  size_t w = root(2 + nf) + 1;  // header, roots, then a count before each array
+  last = w; w += 32 + 1;
+  q = w; w += N_QUERIES + 1;
+  auto paths = [&](uint32_t d) {
+    depth.push_back(d);
+    tree.push_back(w);
+    w += (size_t)2 * N_QUERIES * (1 + 8 * (size_t)d) + 1;
+  };
   tv = w; w += 2 * N_QUERIES;
+  paths(log_eval);
   qv = w; w += 2 * N_QUERIES * 4;
-  fv = w; w += (size_t)nf * 2 * N_QUERIES * 4;
-  depth.push_back(log_eval);
-  depth.push_back(log_eval);
-  for (uint32_t l = 0; l < nf; l++) depth.push_back(log_eval - 1 - l);
-  for (uint32_t d : depth) { tree.push_back(w); w += (size_t)2 * N_QUERIES * d * 8; }
-  words = w;
+  paths(log_eval);
+  w++;  // after the layer count, the first layer's query count
+  for (uint32_t l = 0; l < nf; l++) {
+    fv.push_back(w); w += 2 * N_QUERIES * 4;
+    paths(log_eval - 1 - l);
+  }
+  words = w - 1;  // no count follows the last paths
 }
 
-// KRAK v1 from a host copy of the arena (after the stream completed). The format
-// is a sequence of little-endian u32 words, so on a little-endian host each field
-// is copied as words: the size is known up front and every region is one memcpy.
-static_assert(__BYTE_ORDER__ == __ORDER_LITTLE_ENDIAN__, "KRAK serialisation copies host words as LE bytes");
-void ArenaLayout::serialize(const uint32_t* A, uint32_t a, uint32_t b, std::vector<uint8_t>& out) const {
-  size_t total = 5 + 16 + 1 + 8 * (size_t)nf + 1 + 32 + 1 + N_QUERIES + 1 + 2 * N_QUERIES + 1 + 2 * N_QUERIES * 4 + 1;
-  for (size_t t = 0; t < depth.size(); t++) total += 2 * N_QUERIES * (1 + (size_t)depth[t] * 8);
-  total += (size_t)nf * (1 + 2 * N_QUERIES * 4);
-  out.resize(total * 4);
-  uint8_t* w = out.data();
-  auto w32 = [&](uint32_t v) { std::memcpy(w, &v, 4); w += 4; };
-  auto wn = [&](const uint32_t* p, size_t cnt) { std::memcpy(w, p, cnt * 4); w += cnt * 4; };
-  auto wpaths = [&](size_t off, uint32_t d, uint32_t s) {
-    for (uint32_t qi = 0; qi < N_QUERIES; qi++) { w32(d); wn(A + off + ((size_t)(s * N_QUERIES + qi) * d) * 8, (size_t)d * 8); }
-  };
-  w32(0x4B52414Bu); w32(1); w32(log_n); w32(a); w32(b);
-  wn(A + roots, 16);
-  w32(nf);
-  wn(A + roots + 16, 8 * nf);
-  w32(8);
-  wn(A + last, 32);
-  w32(N_QUERIES);
-  wn(A + q, N_QUERIES);
-  w32(N_QUERIES);
-  wn(A + tv, 2 * N_QUERIES);
-  wpaths(tree[0], depth[0], 0);
-  wpaths(tree[0], depth[0], 1);
-  w32(N_QUERIES);
-  wn(A + qv, 2 * N_QUERIES * 4);
-  wpaths(tree[1], depth[1], 0);
-  wpaths(tree[1], depth[1], 1);
-  w32(nf);
-  for (uint32_t l = 0; l < nf; l++) {
-    w32(N_QUERIES);
-    wn(A + fv + (size_t)l * 2 * N_QUERIES * 4, 2 * N_QUERIES * 4);
-    wpaths(tree[2 + l], depth[2 + l], 0);
-    wpaths(tree[2 + l], depth[2 + l], 1);
-  }
+static_assert(__BYTE_ORDER__ == __ORDER_LITTLE_ENDIAN__, "arena words are KRAK's little-endian words");
+void ArenaLayout::finish(uint8_t* arena, uint32_t a, uint32_t b) const {
+  auto put = [&](size_t at, uint32_t v) { std::memcpy(arena + 4 * at, &v, 4); };
+  put(0, 0x4B52414Bu);
+  put(1, 1);
+  put(2, log_n);
+  put(3, a);
+  put(4, b);
+  put(21, nf);
+  put(last - 1, 8);
+  for (size_t at : {q, tv, qv}) put(at - 1, N_QUERIES);
+  put(fv[0] - 2, nf);
+  for (size_t at : fv) put(at - 1, N_QUERIES);
 }
 
 // ------------------------------------------------------------------ the prover
@@ -434,11 +418,11 @@ struct GraphProver::Impl {
     VS_LAUNCHED("fib_trace_params_kernel");
     VS_TRY(lde_cached(TW_NATIVE, d_trace, 0, d_eval, 0, 1, log_n, BLOWUP_BITS, st));
     VS_TRY(commit(LeafOne{d_eval}, trace_t));
-    ch_mix_draw_kernel<<<1, 32, 0, st>>>(d_ch, 1, trace_t.layers.back(), d_arena + lay.roots, d_alpha);
+    ch_mix_draw_kernel<<<1, 32, 0, st>>>(d_ch, 1, trace_t.layers.back(), d_arena + lay.root(0), d_alpha);
     VS_LAUNCHED("ch_mix_draw_kernel");
     const LeafFibQuotD quot{d_eval, N - 1, d_alpha};
     VS_TRY(commit(quot, quot_t));
-    ch_mix_draw_kernel<<<1, 32, 0, st>>>(d_ch, 0, quot_t.layers.back(), d_arena + lay.roots + 8, d_alpha + 4);
+    ch_mix_draw_kernel<<<1, 32, 0, st>>>(d_ch, 0, quot_t.layers.back(), d_arena + lay.root(1), d_alpha + 4);
     VS_LAUNCHED("ch_mix_draw_kernel");
     for (uint32_t l = 0; l < nf; l++) {
       const uint32_t cur = log_eval - l;
@@ -453,7 +437,7 @@ struct GraphProver::Impl {
                        {fri_vals[l][0], fri_vals[l][1], fri_vals[l][2], fri_vals[l][3]}, tw, a};
         VS_TRY(commit(leaf, fri_t[l]));
       }
-      ch_mix_draw_kernel<<<1, 32, 0, st>>>(d_ch, 0, fri_t[l].layers.back(), d_arena + lay.roots + 8 * (2 + l),
+      ch_mix_draw_kernel<<<1, 32, 0, st>>>(d_ch, 0, fri_t[l].layers.back(), d_arena + lay.root(2 + l),
                                            l + 1 < nf ? d_alpha + 4 * (2 + l) : nullptr);
       VS_LAUNCHED("ch_mix_draw_kernel");
     }
@@ -471,7 +455,7 @@ struct GraphProver::Impl {
     dp.nf = nf;
     for (uint32_t l = 0; l < nf; l++)
       for (int k = 0; k < 4; k++) dp.fri[l][k] = fri_vals[l][k];
-    dp.fri_vals = d_arena + lay.fv;
+    for (uint32_t l = 0; l < nf; l++) dp.fri_vals[l] = d_arena + lay.fv[l];
     decommit_values_kernel<<<1, 2 * N_QUERIES, 0, st>>>(dp);
     VS_LAUNCHED("decommit_values_kernel");
     VS_TRY(paths(LeafOne{d_eval}, trace_t, 0, lay.tree[0]));
@@ -519,7 +503,9 @@ int GraphProver::launch(uint32_t a, uint32_t b, cudaStream_t on) {
 int GraphProver::finish(uint32_t a, uint32_t b, std::vector<uint8_t>& out) {
   VS_CUDA(cudaStreamSynchronize(impl->running ? impl->running : impl->st));
   impl->running = nullptr;  // the launch stream may be reused for other work from here on
-  impl->lay.serialize(impl->h_arena, a, b, out);
+  uint8_t* proof = reinterpret_cast<uint8_t*>(impl->h_arena);
+  impl->lay.finish(proof, a, b);
+  out.assign(proof, proof + impl->lay.bytes());
   return VS_OK;
 }
 bool GraphProver::busy() const {

@@ -8,17 +8,22 @@
 
 namespace vs {
 
-// Proof arena: the words of one proof as the device writes them (roots, last
-// layer, queries, values, authentication paths), serialised to KRAK v1
-// (src/bin/stark_cli.rs:907-976) on the host. Shared by the graph-captured and
-// the batched provers, so both emit the same bytes.
+// Proof arena: one proof as the device writes it, laid out as its KRAK v1 wire form
+// (src/bin/stark_cli.rs:907-976, little-endian words), so that a host copy of the arena
+// is the proof once its header and counts are filled in. Shared by the graph-captured
+// and the batched provers, so both emit the same bytes. A path is its depth, then depth
+// hashes; the device writes it whole.
 struct ArenaLayout {
   uint32_t log_n = 0, log_eval = 0, nf = 0;
-  size_t roots = 0, last = 0, q = 0, tv = 0, qv = 0, fv = 0, words = 0;
+  size_t last = 0, q = 0, tv = 0, qv = 0, words = 0;
+  std::vector<size_t> fv;       // opened values per FRI layer
   std::vector<size_t> tree;     // path region per tree: trace, quotient, FRI layers
   std::vector<uint32_t> depth;  // authentication-path depth per tree
+  size_t root(size_t t) const { return t < 2 ? 5 + 8 * t : 22 + 8 * (t - 2); }  // of tree t
   void plan(uint32_t log_n);
-  void serialize(const uint32_t* arena, uint32_t a, uint32_t b, std::vector<uint8_t>& out) const;
+  size_t bytes() const { return 4 * words; }
+  // The words the device does not write, into a host copy of the arena.
+  void finish(uint8_t* arena, uint32_t a, uint32_t b) const;
 };
 
 // Fibonacci trace of each job y (blockIdx.y): t0 = ab[2y], t1 = ab[2y+1], written
