@@ -1,0 +1,59 @@
+"""LDEs and transforms in both conventions on either side of the rules that run jobs of few
+words in the small-job passes, against the oracle."""
+import numpy as np
+import pytest
+
+from gpu_util import dev, empty, host, ptr, ptr_array, rand_m31, u32_host
+
+pytestmark = pytest.mark.gpu
+
+import oracle_lib as O  # noqa: E402
+import vortexstark_b200 as V  # noqa: E402
+
+
+def cases():
+    for log_n in range(5, 14):
+        for blowup in (0, 1, 3):
+            yield log_n, blowup, 3
+    yield 13, 3, 64   # 2^22 evaluation words: the most of at most 13 layers
+    yield 13, 3, 65   # above 2^22 evaluation words
+    yield 8, 4, 2     # more blocks than it takes
+    yield 14, 2, 16   # 2^20 evaluation words: the most of a larger transform
+    yield 14, 2, 17
+    yield 16, 1, 3    # lower and upper passes, clusters of two
+    yield 17, 3, 1    # and of eight
+    yield 19, 1, 1
+    yield 19, 0, 2
+
+
+@pytest.mark.parametrize("log_n,blowup,n_cols", list(cases()))
+def test_small_lde(log_n, blowup, n_cols):
+    n, N = 1 << log_n, 1 << (log_n + blowup)
+    cols = rand_m31(np.random.default_rng(log_n * 100 + blowup), n_cols, n)
+    dst = empty(n_cols * N)
+    V.check(V.lib().vs_lde_stwo(ptr(dev(cols.reshape(-1))), n, ptr(dst), N, n_cols, log_n, blowup, None), "vs_lde_stwo")
+    assert np.array_equal(host(dst).reshape(n_cols, N), O.stwo_lde_columns(cols, log_n, blowup, threads=8))
+    V.check(V.lib().vs_lde_native(ptr(dev(cols[0])), 0, ptr(dst), 0, 1, log_n, blowup, None), "vs_lde_native")
+    coeffs = O.native_interpolate(cols[0], log_n)
+    exp = O.native_evaluate(np.concatenate([coeffs, np.zeros(N - n, np.uint32)]), log_n + blowup)
+    assert np.array_equal(host(dst)[:N], exp)
+
+
+@pytest.mark.parametrize("log_n", list(range(5, 21)))
+def test_small_transforms(log_n):
+    """2^19 words and fewer take the small-job passes, in place, single and batched."""
+    L = V.lib()
+    x = rand_m31(np.random.default_rng(log_n), 1 << log_n)
+    fwd, inv = O.stwo_twiddles(log_n)
+    d, tf, ti = dev(x), dev(fwd), dev(inv)
+    L.cuda_stwo_ntt_evaluate(ptr(d), ptr(tf), 1 << log_n)
+    assert np.array_equal(host(d), O.stwo_evaluate(x, log_n))
+    L.cuda_stwo_ntt_interpolate(ptr(d), ptr(ti), 1 << log_n)
+    assert np.array_equal(host(d), x)
+    cols = [dev(x), dev(x[::-1].copy())]
+    tw = O.native_twiddles(log_n)
+    arr, line, circle = ptr_array(cols), dev(tw["line"]), dev(tw["circle"])
+    L.cuda_circle_ntt_evaluate_batch(ptr(arr), ptr(line), ptr(circle), u32_host(tw["offsets"]), u32_host(tw["sizes"]),
+                                     log_n - 1, 1 << log_n, 2)
+    for c, v in zip(cols, (x, x[::-1])):
+        assert np.array_equal(host(c), O.native_evaluate(v.copy(), log_n))

@@ -393,6 +393,232 @@ __global__ void __launch_bounds__(1 << (M + C - 5), 2) ntt_lde_top_kernel(NttPas
   }
 }
 
+// Thread-block cluster primitives (the LDE top pass's cluster form): split cluster
+// barrier (arrive with release, wait with acquire semantics at cluster scope) and
+// loads from a peer CTA's shared memory (distributed shared memory).
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+// Arrive without release semantics (it does not wait for the thread's outstanding
+// stores): for arrivals that only announce that the thread's reads are complete,
+// which program order already guarantees when each loaded value has been consumed
+// by an instruction before the arrive.
+__device__ __forceinline__ void cluster_arrive_relaxed() {
+  asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+__device__ __forceinline__ uint32_t cluster_rank() {
+  uint32_t r;
+  asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+// the same shared-memory offset in the CTA of cluster rank `rank`
+__device__ __forceinline__ uint32_t cluster_peer(uint32_t saddr, uint32_t rank) {
+  uint32_t r;
+  asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(saddr), "r"(rank));
+  return r;
+}
+__device__ __forceinline__ uint4 ld_cluster16(uint32_t addr) {
+  uint4 v;
+  asm volatile("ld.shared::cluster.v4.u32 {%0, %1, %2, %3}, [%4];"
+               : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
+               : "r"(addr)
+               : "memory");
+  return v;
+}
+
+// ---- Passes of small jobs: eight words a thread.
+// Where the 8192-word tiles of all columns are fewer than a wave, a pass takes as long as
+// one tile does: eight rounds' worth of work on 32 words a thread. These tiles of at most
+// 2^13 words give each thread eight words and rounds of three layers, so that the same
+// columns are many more, shorter CTAs. The first round reads and the last writes global
+// memory directly; what bounds a tile is the latency of the exchanges between rounds.
+// Twiddles are fetched one round ahead.
+// T = M + C tile bits, layers over bits [C, T) as in Tile.
+template <int M, int C>
+struct Small {
+  static constexpr int T = M + C, NT = 1 << (T - 3), NR = (M + 2) / 3;
+  static constexpr int P0(int r) { return C + 3 * r; }
+  static constexpr int R(int r) { return 3 * (r + 1) <= M ? 3 : M - 3 * r; }
+  static constexpr uint32_t BYTES = (9u << T) / 8 * 4;
+};
+// Eight words of padding per 64 spread the rounds of the low bits over the banks and keep
+// 16-byte chunks whole.
+__device__ __forceinline__ uint32_t small_at(uint32_t a) { return a + ((a >> 6) << 3); }
+// Doubled twiddles of round r: layer q of subgroup s at t[s * (K - 1) + K - (K >> q) + gg].
+template <int M, int C, int r>
+__device__ __forceinline__ void small_tw(uint32_t (&t)[8], const TileGeo& g, const NttTw& tw) {
+  using S = Small<M, C>;
+  constexpr int P0 = S::P0(r), R = S::R(r), K = 1 << R, SUB = 1 << (3 - R);
+#pragma unroll
+  for (int s = 0; s < SUB; s++) {
+    const uint32_t base = ins<P0, R>(threadIdx.x + s * S::NT, 0);
+#pragma unroll
+    for (int q = 0; q < R; q++) {
+      const int p = P0 + q, cnt = K >> (q + 1), o = s * (K - 1) + K - (K >> q);
+      const uint32_t hb = (g.hi << (S::T - 1 - p)) | (base >> (p + 1));
+      const uint32_t* tp = tw.layer[g.a + p - C] + hb;
+      if (p == 0 && tw.stwo && g.a == 0) {  // [y, -y, -x, x] of one pair of line layer 0
+        const uint2 w = __ldg(reinterpret_cast<const uint2*>(tw.flat) + (hb >> 2));
+        t[o] = w.y << 1;
+        t[o + 1] = neg(w.y) << 1;
+        t[o + 2] = neg(w.x) << 1;
+        t[o + 3] = w.x << 1;
+      } else if (cnt == 4) {
+        const uint4 w = __ldg(reinterpret_cast<const uint4*>(tp));
+        t[o] = w.x << 1;
+        t[o + 1] = w.y << 1;
+        t[o + 2] = w.z << 1;
+        t[o + 3] = w.w << 1;
+      } else if (cnt == 2) {
+        const uint2 w = __ldg(reinterpret_cast<const uint2*>(tp));
+        t[o] = w.x << 1;
+        t[o + 1] = w.y << 1;
+      } else {
+        t[o] = __ldg(tp) << 1;
+      }
+    }
+  }
+}
+template <bool FWD, int M, int C, int r>
+__device__ __forceinline__ void small_bfly(uint32_t (&v)[8], const uint32_t (&t)[8]) {
+  constexpr int R = Small<M, C>::R(r), K = 1 << R, SUB = 1 << (3 - R);
+#pragma unroll
+  for (int s = 0; s < SUB; s++)
+#pragma unroll
+    for (int qq = 0; qq < R; qq++) {
+      const int q = FWD ? R - 1 - qq : qq;
+#pragma unroll
+      for (int gg = 0; gg < (K >> (q + 1)); gg++)
+#pragma unroll
+        for (int l = 0; l < (1 << q); l++) {
+          const int k0 = s * K + ((gg << (q + 1)) | l);
+          bfly<FWD>(v[k0], v[k0 + (1 << q)], t[s * (K - 1) + K - (K >> q) + gg]);
+        }
+    }
+}
+// The thread's words of round r: to or from the padded tile, or global memory (whose
+// element e of the tile is at at(e); a C = 0 tile's round 0 is eight consecutive words).
+template <int M, int C, int r, bool STORE, class At>
+__device__ __forceinline__ void small_move(uint32_t (&v)[8], const At& at) {
+  using S = Small<M, C>;
+  constexpr int P0 = S::P0(r), R = S::R(r), K = 1 << R, SUB = 1 << (3 - R);
+  if constexpr (C == 0 && r == 0) {
+    static_assert(R == 3, "tiles of at least three layers");
+    uint4* p = reinterpret_cast<uint4*>(at(8 * threadIdx.x));
+    if (STORE) {
+      p[0] = make_uint4(v[0], v[1], v[2], v[3]);
+      p[1] = make_uint4(v[4], v[5], v[6], v[7]);
+    } else {
+      const uint4 a = p[0], b = p[1];
+      v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
+      v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
+    }
+  } else {
+#pragma unroll
+    for (int s = 0; s < SUB; s++)
+#pragma unroll
+      for (int k = 0; k < K; k++) {
+        uint32_t* p = at(ins<P0, R>(threadIdx.x + s * S::NT, k));
+        if (STORE) *p = v[s * K + k];
+        else v[s * K + k] = *p;
+      }
+  }
+}
+// Round r's words to round rn's through the tile.
+template <int M, int C, int r, int rn>
+__device__ __forceinline__ void small_exchange(uint32_t (&v)[8], uint32_t* sm) {
+  auto at = [&](uint32_t e) { return sm + small_at(e); };
+  small_move<M, C, r, true>(v, at);
+  __syncthreads();
+  small_move<M, C, rn, false>(v, at);
+  __syncthreads();
+}
+// Inverse rounds r.. (round r's words in v, twiddles in t); ends with the top round's words in
+// v and, with NEXT, the first twiddles of the forward rounds over (gf, tf) in t.
+template <int M, int C, int r, bool NEXT>
+__device__ __forceinline__ void small_inv(uint32_t (&v)[8], uint32_t (&t)[8], uint32_t* sm, const TileGeo& g,
+                                          const NttTw& tw, const TileGeo& gf, const NttTw& tf) {
+  constexpr bool TOP = r + 1 == Small<M, C>::NR;
+  uint32_t tn[8];
+  if constexpr (!TOP) small_tw<M, C, (TOP ? 0 : r + 1)>(tn, g, tw);
+  else if constexpr (NEXT) small_tw<M, C, r>(tn, gf, tf);
+  small_bfly<false, M, C, r>(v, t);
+  if constexpr (!TOP || NEXT) {
+#pragma unroll
+    for (int k = 0; k < 8; k++) t[k] = tn[k];
+  }
+  if constexpr (!TOP) {
+    small_exchange<M, C, r, (TOP ? 0 : r + 1)>(v, sm);
+    small_inv<M, C, (TOP ? 0 : r + 1), NEXT>(v, t, sm, g, tw, gf, tf);
+  }
+}
+template <int M, int C, int r>
+__device__ __forceinline__ void small_fwd(uint32_t (&v)[8], uint32_t (&t)[8], uint32_t* sm, const TileGeo& g,
+                                          const NttTw& tw) {
+  uint32_t tn[8];
+  if constexpr (r > 0) small_tw<M, C, (r > 0 ? r - 1 : 0)>(tn, g, tw);
+  small_bfly<true, M, C, r>(v, t);
+  if constexpr (r > 0) {
+#pragma unroll
+    for (int k = 0; k < 8; k++) t[k] = tn[k];
+    small_exchange<M, C, r, (r > 0 ? r - 1 : 0)>(v, sm);
+    small_fwd<M, C, (r > 0 ? r - 1 : 0)>(v, t, sm, g, tw);
+  }
+}
+template <bool FWD, int M, int C>
+__global__ void __launch_bounds__(Small<M, C>::NT) ntt_pass_small_kernel(NttPass p, uint32_t n_cols) {
+  extern __shared__ __align__(16) uint32_t small_sm[];
+  constexpr int TOP = Small<M, C>::NR - 1, FIRST = FWD ? TOP : 0, LAST = FWD ? 0 : TOP;
+  const uint32_t col = blockIdx.x % n_cols;
+  const TileGeo g = tile_geo<M, C>(p.a, blockIdx.x / n_cols);
+  uint32_t v[8], t[8];
+  uint32_t* src = const_cast<uint32_t*>(col_src(p, col));
+  small_move<M, C, FIRST, false>(v, [&](uint32_t e) { return src + gidx<M, C>(g, e); });
+  small_tw<M, C, FIRST>(t, g, p.tw);
+  if constexpr (FWD) {
+    small_fwd<M, C, TOP>(v, t, small_sm, g, p.tw);
+  } else {
+    small_inv<M, C, 0, false>(v, t, small_sm, g, p.tw, g, p.tw);
+    if (p.scale) {
+#pragma unroll
+      for (int k = 0; k < 8; k++) v[k] = mul(v[k], p.scale);
+    }
+  }
+  uint32_t* dst = col_dst(p, col);
+  small_move<M, C, LAST, true>(v, [&](uint32_t e) { return dst + gidx<M, C>(g, e); });
+}
+// The LDE's top pass in this form: one CTA per (tile, column, blowup block), each doing the
+// inverse layers for itself; its coefficients stay in registers, since the top round of
+// the inverse layers and the first of the forward ones hold the same words. A whole
+// transform (C = 0, M <= 13) is one such pass. The blocks' CTAs of a tile are a cluster
+// (grid y): block 0 is written over the tile that they all read, so none stores before all
+// have read it.
+template <int M, int C>
+__global__ void __launch_bounds__(Small<M, C>::NT) ntt_lde_top_small_kernel(NttPass inv, NttPass fwd, uint32_t n_cols) {
+  extern __shared__ __align__(16) uint32_t small_sm[];
+  constexpr int TOP = Small<M, C>::NR - 1;
+  const uint32_t col = blockIdx.x % n_cols, q = blockIdx.y;
+  const TileGeo gi = tile_geo<M, C>(inv.a, blockIdx.x / n_cols);
+  TileGeo gf = gi;
+  gf.hi = q;
+  gf.gbase = (q << (gi.a + M)) | gi.gbase;
+  uint32_t v[8], t[8];
+  uint32_t* src = const_cast<uint32_t*>(col_src(inv, col));
+  small_move<M, C, 0, false>(v, [&](uint32_t e) { return src + gidx<M, C>(gi, e); });
+  small_tw<M, C, 0>(t, gi, inv.tw);
+  small_inv<M, C, 0, true>(v, t, small_sm, gi, inv.tw, gf, fwd.tw);
+  cluster_arrive();  // this thread's words of the tile are read
+#pragma unroll
+  for (int k = 0; k < 8; k++) v[k] = mul(v[k], inv.scale);
+  if (inv.dst && q == 0) {  // the caller keeps the coefficients too
+    uint32_t* cd = col_dst(inv, col);
+    small_move<M, C, TOP, true>(v, [&](uint32_t e) { return cd + gidx<M, C>(gi, e); });
+  }
+  small_fwd<M, C, TOP>(v, t, small_sm, gf, fwd.tw);
+  cluster_wait();
+  uint32_t* dst = col_dst(fwd, col);
+  small_move<M, C, 0, true>(v, [&](uint32_t e) { return dst + gidx<M, C>(gf, e); });
+}
+
 // ---- Chunk-round variant of the fused LDE top pass (tiles with C >= 2).
 // A thread holds eight 16-byte chunks (the four words of tile bits 0-1) along
 // three round bits, so every shared-memory access is 128-bit, and the four words
@@ -437,38 +663,6 @@ __host__ __device__ constexpr bool warp_local_word() {
 __device__ __forceinline__ void round_sync(bool warp_local) {
   if (warp_local) __syncwarp();
   else __syncthreads();
-}
-
-// Thread-block cluster primitives (the LDE top pass's cluster form): split cluster
-// barrier (arrive with release, wait with acquire semantics at cluster scope) and
-// loads from a peer CTA's shared memory (distributed shared memory).
-__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
-// Arrive without release semantics (it does not wait for the thread's outstanding
-// stores): for arrivals that only announce that the thread's reads are complete,
-// which program order already guarantees when each loaded value has been consumed
-// by an instruction before the arrive.
-__device__ __forceinline__ void cluster_arrive_relaxed() {
-  asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
-}
-__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
-__device__ __forceinline__ uint32_t cluster_rank() {
-  uint32_t r;
-  asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-  return r;
-}
-// the same shared-memory offset in the CTA of cluster rank `rank`
-__device__ __forceinline__ uint32_t cluster_peer(uint32_t saddr, uint32_t rank) {
-  uint32_t r;
-  asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(saddr), "r"(rank));
-  return r;
-}
-__device__ __forceinline__ uint4 ld_cluster16(uint32_t addr) {
-  uint4 v;
-  asm volatile("ld.shared::cluster.v4.u32 {%0, %1, %2, %3}, [%4];"
-               : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
-               : "r"(addr)
-               : "memory");
-  return v;
 }
 
 // Word address of chunk k (R round bits at word bit P0) of chunk group o; o
@@ -735,6 +929,10 @@ __global__ void __launch_bounds__(1 << (M + C - 5), 3) ntt_lde_top4_kernel(NttPa
   // each block's first-round twiddles are fetched right after the butterflies of
   // the round before it (the last inverse round, then each block's round 0)
   inv_rounds4<M, C, 0>(sm, cf, gi, inv.tw, inv.scale, t, gf, fwd.tw);
+  if (inv.dst) {  // the caller keeps the coefficients too
+    __syncthreads();
+    tile_store4<M, C>(cf, col_dst(inv, blockIdx.y), gi);
+  }
   if constexpr (K > 1) cluster_arrive_relaxed();  // this CTA's last reads of sm are consumed
   for (uint32_t q = 0; q < (1u << B); q++) {
     const TileGeo gq = gf;
@@ -916,6 +1114,29 @@ template <int M> TopFn top_hi() { return ntt_lde_top4_kernel<M, 13 - M>; }
 constexpr int kTopPair = 2;
 TopFn top_hi_pair() { return ntt_lde_top4_kernel<11, 2, kTopPair>; }
 template <int M> TopFn top5_hi() { return ntt_lde_top_kernel<M, 13 - M>; }
+// Small-job passes: whole transforms and lower passes (C = 0), upper passes of 7-9 layers
+// with 32-byte tile rows.
+constexpr uint32_t kSmallMaxL = 19, kSmallUpperC = 3;
+using SmallFn = void (*)(NttPass, uint32_t);
+using SmallTopFn = void (*)(NttPass, NttPass, uint32_t);
+#define VS_SMALL_LO VS_SM(5, 0) VS_SM(6, 0) VS_SM(7, 0) VS_SM(8, 0) VS_SM(9, 0) VS_SM(10, 0) VS_SM(11, 0) VS_SM(12, 0) VS_SM(13, 0)
+#define VS_SMALL_HI VS_SM(7, 3) VS_SM(8, 3) VS_SM(9, 3)
+static SmallFn small_fn(bool fwd, uint32_t M, uint32_t C) {
+  switch (16 * M + C) {
+#define VS_SM(m, c) case 16 * m + c: return fwd ? (SmallFn)ntt_pass_small_kernel<true, m, c> : ntt_pass_small_kernel<false, m, c>;
+    VS_SMALL_LO VS_SMALL_HI
+#undef VS_SM
+    default: return nullptr;
+  }
+}
+static SmallTopFn small_top_fn(uint32_t M, uint32_t C) {
+  switch (16 * M + C) {
+#define VS_SM(m, c) case 16 * m + c: return ntt_lde_top_small_kernel<m, c>;
+    VS_SMALL_LO VS_SMALL_HI
+#undef VS_SM
+    default: return nullptr;
+  }
+}
 
 static PassFn pass_fn(bool fwd, uint32_t M, uint32_t C) {
 #define VS_LO(m) case m: return fwd ? pass_lo<true, m>() : pass_lo<false, m>();
@@ -989,6 +1210,32 @@ __global__ void scale_kernel(uint32_t* __restrict__ d, uint32_t s, uint32_t n) {
 // ------------------------------------------------------------------ host side
 static const uint32_t kMaxT = 13;  // tile of 8192 words (32 KiB), 256 threads
 static const uint32_t kMinC = 2;   // >= 16-byte contiguous runs per tile row
+// Jobs of few words (all columns together) run in the small-job passes unless a plan was
+// set for their size. Measured (us, 8192-word tiles then small-job passes):
+//  * transforms: 2^14 21.6 -> 17.1, 2^19 23.9 -> 20.5, but 2^20 23.9 -> 25.7;
+//  * LDEs of at most 13 layers, by evaluation words: 34 x 2^10 x4 (2^17) 16.8 -> 7.5,
+//    34 x 2^13 x8 (2^21) 43.5 -> 22.9;
+//  * LDEs above: 2 x 2^14 x4 24.9 -> 17.1, 4 x 2^16 x4 (2^20) 27.0 -> 22.9, 2 x 2^18 x2
+//    (2^20) 25.7 -> 23.0, but 7 x 2^17 x2 (1.75 x 2^20) 29.1 -> 29.2 and 34 x 2^14 x2
+//    (1.06 x 2^20) 23.0 -> 25.0: the repeated inverse layers then cost more than the
+//    idle SMs they fill.
+static bool default_plan(uint32_t L) {
+  const NttPlan p = ntt_plan(L);
+  return p.lower == 0 && p.items == 0 && p.radix == 3;
+}
+static bool small_transform_job(uint32_t L, uint64_t words) {
+  return L >= 5 && L <= kSmallMaxL && words <= (1ull << 19) && default_plan(L);
+}
+static bool small_lde_job(uint32_t l, uint32_t B, uint32_t n_cols) {
+  const uint64_t words = (uint64_t)n_cols << (l + B);
+  return l >= 5 && l <= kSmallMaxL && B <= 3 && words <= (l <= 13 ? 1ull << 22 : 1ull << 20) && default_plan(l);
+}
+// Lower (C = 0) and upper pass of a small transform of L layers; one pass up to 13.
+static std::vector<PassRange> small_passes(uint32_t L) {
+  if (L <= 13) return {{0, L - 1, 0}};
+  const uint32_t lo = (L + 1) / 2;
+  return {{0, lo - 1, 0}, {lo, L - 1, kSmallUpperC}};
+}
 
 // Per-size plans (process wide). Sizes 14..24 may move layers between the lower
 // pass and the single upper pass: lower in [max(5, L - 11), 13] keeps the upper
@@ -1089,8 +1336,13 @@ static uint32_t persistent_grid(const void* fn, uint32_t threads, uint32_t smem)
   return g;
 }
 
-static int launch_pass(NttPass p, bool fwd, uint32_t n_cols, cudaStream_t st) {
+static int launch_pass(NttPass p, bool fwd, uint32_t n_cols, cudaStream_t st, bool small = false) {
   const uint32_t M = p.b - p.a + 1, T = M + p.c;
+  if (small) {
+    small_fn(fwd, M, p.c)<<<n_cols << (p.log_n - T), 1u << (T - 3), (9u << T) / 8 * 4, st>>>(p, n_cols);
+    VS_LAUNCHED("ntt_pass_small_kernel");
+    return VS_OK;
+  }
   if (p.radix != 5 && p.c == 0 && M == kMaxT && p.items <= 1) {  // one tile per CTA: single-buffered kernel
     PassFn f = fwd ? ntt_pass4s_kernel<true, kMaxT, 0> : ntt_pass4s_kernel<false, kMaxT, 0>;
     const uint64_t tot = (uint64_t)n_cols << (p.log_n - T);
@@ -1249,7 +1501,8 @@ static int ntt_transform_aligned(const NttColumns& io, uint32_t L, const NttTw& 
     return VS_OK;
   }
   const NttPlan plan = ntt_plan(L);
-  auto passes = plan_passes(L, plan.lower);
+  const bool small = small_transform_job(L, (uint64_t)io.n_cols << L);
+  const auto passes = small ? small_passes(L) : plan_passes(L, plan.lower);
   const size_t np = passes.size();
   for (size_t i = 0; i < np; i++) {
     const PassRange& r = fwd ? passes[np - 1 - i] : passes[i];
@@ -1270,23 +1523,30 @@ static int ntt_transform_aligned(const NttColumns& io, uint32_t L, const NttTw& 
     p.dst_cols = io.dst_cols;
     p.dst_stride = io.dst_stride;
     p.scale = (!fwd && i == np - 1) ? inv_n_scale(L) : 0;
-    VS_TRY(launch_pass(p, fwd, io.n_cols, st));
+    VS_TRY(launch_pass(p, fwd, io.n_cols, st, small));
   }
   return VS_OK;
 }
 
 static int ntt_lde_aligned(const NttColumns& io, uint32_t l, uint32_t B, const NttTw& tw_inv, const NttTw& tw_fwd,
-                           cudaStream_t st);
+                           cudaStream_t st, uint32_t* coeffs = nullptr, uint64_t coeffs_stride = 0);
 
 int ntt_lde(const NttColumns& io, uint32_t l, uint32_t B, const NttTw& tw_inv, const NttTw& tw_fwd,
-            cudaStream_t st) {
+            cudaStream_t st, uint32_t* coeffs, uint64_t coeffs_stride) {
   if (l < 5) return set_error(VS_ERR_INVALID, "LDE needs log_n >= 5 (got %u)", l);
   if (io.src_cols || io.dst_cols) return set_error(VS_ERR_INVALID, "LDE takes strided columns");
   StreamScratch tmp(st);
   NttTw ti, tf;
   VS_TRY(aligned_twiddles(tw_inv, l, st, tmp, &ti));
   VS_TRY(aligned_twiddles(tw_fwd, l + B, st, tmp, &tf));
-  if (strided_aligned(io)) return ntt_lde_aligned(io, l, B, ti, tf, st);
+  // The chunk-round top pass has the coefficients in hand and stores them as well;
+  // otherwise they are one more interpolation.
+  const NttColumns cio{io.src, coeffs, nullptr, nullptr, io.src_stride, coeffs_stride, io.n_cols};
+  const bool with = coeffs && (l > kMaxT || small_lde_job(l, B, io.n_cols)) && ntt_plan(l).radix != 5 &&
+                    strided_aligned(cio) && strided_aligned(io);
+  if (coeffs && !with) VS_TRY(ntt_transform(cio, l, ti, false, st));
+  if (strided_aligned(io))
+    return ntt_lde_aligned(io, l, B, ti, tf, st, with ? coeffs : nullptr, coeffs_stride);
   const uint64_t n = 1ull << l, N = n << B;
   uint32_t *S = nullptr, *D = nullptr;
   VS_TRY(tmp.alloc(&S, n * io.n_cols));
@@ -1301,9 +1561,10 @@ int ntt_lde(const NttColumns& io, uint32_t l, uint32_t B, const NttTw& tw_inv, c
 }
 
 static int ntt_lde_aligned(const NttColumns& io, uint32_t l, uint32_t B, const NttTw& tw_inv, const NttTw& tw_fwd,
-                           cudaStream_t st) {
+                           cudaStream_t st, uint32_t* coeffs, uint64_t coeffs_stride) {
   const NttPlan plan = ntt_plan(l);
-  auto passes = plan_passes(l, plan.lower);
+  const bool small = small_lde_job(l, B, io.n_cols);
+  const auto passes = small ? small_passes(l) : plan_passes(l, plan.lower);
   const size_t np = passes.size();
   // 1. inverse passes below the top one: src -> dst[0, n)
   for (size_t i = 0; i + 1 < np; i++) {
@@ -1320,7 +1581,7 @@ static int ntt_lde_aligned(const NttColumns& io, uint32_t l, uint32_t B, const N
     p.src_stride = i == 0 ? io.src_stride : io.dst_stride;
     p.dst = io.dst;
     p.dst_stride = io.dst_stride;
-    VS_TRY(launch_pass(p, false, io.n_cols, st));
+    VS_TRY(launch_pass(p, false, io.n_cols, st, small));
   }
   // 2. fused top pass
   {
@@ -1340,39 +1601,58 @@ static int ntt_lde_aligned(const NttColumns& io, uint32_t l, uint32_t B, const N
     pf.log_n = l + B;
     pf.dst = io.dst;
     pf.dst_stride = io.dst_stride;
+    pi.dst = coeffs;
+    pi.dst_stride = coeffs_stride;
     const uint32_t M = r.b - r.a + 1, T = M + r.c;
-    TopFn fn = top_fn(M, r.c, plan.radix);
-    if (!fn) return set_error(VS_ERR_INVALID, "ntt: no LDE kernel for shape M=%u C=%u", M, r.c);
-    const uint32_t smem = 8u << T;  // working tile + coefficient tile
-    const dim3 grid(1u << (l - T), io.n_cols), block(1u << (T - 5));
-    // 16-byte-row tiles run as CTA pairs (whole-sector tile stores); if the
-    // cluster launch is refused, the plain kernel runs instead
-    TopFn cfn = nullptr;
-    const uint32_t K = kTopPair;
-    if (plan.radix != 5 && M == 11 && r.c == 2) cfn = top_hi_pair();
-    bool launched = false;
-    if (cfn && grid.x % K == 0) {
-      VS_TRY(allow_smem((const void*)cfn, smem));
+    if (small) {
       cudaLaunchConfig_t cfg = {};
-      cfg.gridDim = grid;
-      cfg.blockDim = block;
-      cfg.dynamicSmemBytes = smem;
+      cfg.gridDim = dim3(io.n_cols << (l - T), 1u << B);
+      cfg.blockDim = 1u << (T - 3);
+      cfg.dynamicSmemBytes = (9u << T) / 8 * 4;
       cfg.stream = st;
       cudaLaunchAttribute attr[1];
       attr[0].id = cudaLaunchAttributeClusterDimension;
-      attr[0].val.clusterDim.x = K;
-      attr[0].val.clusterDim.y = 1;
+      attr[0].val.clusterDim.x = 1;
+      attr[0].val.clusterDim.y = 1u << B;
       attr[0].val.clusterDim.z = 1;
       cfg.attrs = attr;
       cfg.numAttrs = 1;
-      if (cudaLaunchKernelEx(&cfg, cfn, pi, pf, B) == cudaSuccess) launched = true;
-      else cudaGetLastError();  // clear the refused launch's error
+      VS_CUDA(cudaLaunchKernelEx(&cfg, small_top_fn(M, r.c), pi, pf, io.n_cols));
+      VS_LAUNCHED("ntt_lde_top_small_kernel");
+    } else {
+      TopFn fn = top_fn(M, r.c, plan.radix);
+      if (!fn) return set_error(VS_ERR_INVALID, "ntt: no LDE kernel for shape M=%u C=%u", M, r.c);
+      const uint32_t smem = 8u << T;  // working tile + coefficient tile
+      const dim3 grid(1u << (l - T), io.n_cols), block(1u << (T - 5));
+      // 16-byte-row tiles run as CTA pairs (whole-sector tile stores); if the
+      // cluster launch is refused, the plain kernel runs instead
+      TopFn cfn = nullptr;
+      const uint32_t K = kTopPair;
+      if (plan.radix != 5 && M == 11 && r.c == 2) cfn = top_hi_pair();
+      bool launched = false;
+      if (cfn && grid.x % K == 0) {
+        VS_TRY(allow_smem((const void*)cfn, smem));
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = grid;
+        cfg.blockDim = block;
+        cfg.dynamicSmemBytes = smem;
+        cfg.stream = st;
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = K;
+        attr[0].val.clusterDim.y = 1;
+        attr[0].val.clusterDim.z = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+        if (cudaLaunchKernelEx(&cfg, cfn, pi, pf, B) == cudaSuccess) launched = true;
+        else cudaGetLastError();  // clear the refused launch's error
+      }
+      if (!launched) {
+        VS_TRY(allow_smem((const void*)fn, smem));
+        fn<<<grid, block, smem, st>>>(pi, pf, B);
+      }
+      VS_LAUNCHED("ntt_lde_top_kernel");
     }
-    if (!launched) {
-      VS_TRY(allow_smem((const void*)fn, smem));
-      fn<<<grid, block, smem, st>>>(pi, pf, B);
-    }
-    VS_LAUNCHED("ntt_lde_top_kernel");
   }
   // 3. forward passes below the top one over the whole evaluation domain
   for (int i = (int)np - 2; i >= 0; i--) {
@@ -1389,7 +1669,7 @@ static int ntt_lde_aligned(const NttColumns& io, uint32_t l, uint32_t B, const N
     p.src_stride = io.dst_stride;
     p.dst = io.dst;
     p.dst_stride = io.dst_stride;
-    VS_TRY(launch_pass(p, true, io.n_cols, st));
+    VS_TRY(launch_pass(p, true, io.n_cols, st, small));
   }
   return VS_OK;
 }
@@ -1432,7 +1712,7 @@ int tw_for(int kind, uint32_t L, bool forward, NttTw* out, cudaStream_t st) {
 }
 
 int lde_cached(int kind, const uint32_t* src, uint64_t src_stride, uint32_t* dst, uint64_t dst_stride,
-               uint32_t n_cols, uint32_t l, uint32_t B, cudaStream_t st) {
+               uint32_t n_cols, uint32_t l, uint32_t B, cudaStream_t st, uint32_t* coeffs, uint64_t coeffs_stride) {
   if (!src || !dst || n_cols == 0) return set_error(VS_ERR_INVALID, "lde: null argument");
   if (l < 2 || l + B > 30) return set_error(VS_ERR_INVALID, "lde: log_n %u + blowup %u out of range", l, B);
   NttTw ti, tf;
@@ -1446,12 +1726,14 @@ int lde_cached(int kind, const uint32_t* src, uint64_t src_stride, uint32_t* dst
       VS_CUDA(cudaMemsetAsync(d + n, 0, (N - n) * 4, st));
       NttColumns a{d, d, nullptr, nullptr, 0, 0, 1};
       VS_TRY(ntt_transform(a, l, ti, false, st));
+      if (coeffs)
+        VS_CUDA(cudaMemcpyAsync(coeffs + c * coeffs_stride, d, n * 4, cudaMemcpyDeviceToDevice, st));
       VS_TRY(ntt_transform(a, l + B, tf, true, st));
     }
     return VS_OK;
   }
   NttColumns io{src, dst, nullptr, nullptr, src_stride, dst_stride, n_cols};
-  return ntt_lde(io, l, B, ti, tf, st);
+  return ntt_lde(io, l, B, ti, tf, st, coeffs, coeffs_stride);
 }
 
 // ------------------------------------------------------------------ bit reversal
