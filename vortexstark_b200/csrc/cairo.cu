@@ -17,11 +17,11 @@
 #include <utility>
 #include <vector>
 
-#include "fri.h"
 #include "host_math.h"
 #include "merkle.h"
 #include "ntt.h"
 #include "quotient.h"
+#include "transcript_tree.cuh"
 #include "twiddles.h"
 #include "vs_common.cuh"
 #include "vs_field.cuh"
@@ -509,9 +509,37 @@ h::Q pi_x(h::Q x) {  // 2x^2 - 1
 }
 }  // namespace
 
-// out[c * np + p] = column c (2^L stwo coefficients) at point p; synchronises st.
-int eval_at_points(const uint32_t* const* h_cols, uint32_t n_cols, uint32_t L, const h::Q (*pts)[2], uint32_t np,
-                   h::Q* out, cudaStream_t st) {
+// Columns (2^L stwo coefficients each) at np points: the partial sums of every column and
+// point, left on the device until they are read back together.
+struct EvPartials {
+  uint32_t n_cols = 0, np = 0, gx = 0;  // gx partials a column
+  uint32_t* d = nullptr;
+  uint64_t words() const { return (uint64_t)n_cols * gx * np * 4; }
+  // out[c * np + p] from a host copy of the partials
+  void sum(const uint32_t* h, h::Q* out) const {
+    for (uint32_t i = 0; i < n_cols * np; i++) {
+      const uint32_t c = i / np, p = i % np;
+      h::Q acc{{0, 0, 0, 0}};
+      for (uint32_t b = 0; b < gx; b++) {
+        const uint32_t* v = &h[(((uint64_t)c * gx + b) * np + p) * 4];
+        acc = h::qadd(acc, h::Q{{v[0], v[1], v[2], v[3]}});
+      }
+      out[i] = acc;
+    }
+  }
+};
+EvPartials ev_shape(uint32_t n_cols, uint32_t L, uint32_t np) {
+  EvPartials e;
+  e.n_cols = n_cols;
+  e.np = np;
+  const uint32_t hi_n = 1u << (L - std::min<uint32_t>(L, EV_LOG_SEG));
+  e.gx = n_cols ? std::max<uint32_t>(1, std::min<uint32_t>((hi_n + EV_UNROLL - 1) / EV_UNROLL, (uint32_t)sm_count() * 4 / n_cols)) : 0;
+  return e;
+}
+// Enqueues the kernels that fill e.d (e.words() words).
+int eval_enqueue(const uint32_t* const* h_cols, uint32_t L, const h::Q (*pts)[2], const EvPartials& e, Scratch& s) {
+  cudaStream_t st = s.st;
+  const uint32_t n_cols = e.n_cols, np = e.np;
   if (np == 0 || np > EV_MAX_POINTS) return set_error(VS_ERR_INVALID, "eval_at_points: 1 or 2 points");
   if (L > 30) return set_error(VS_ERR_INVALID, "eval_at_points: log length %u", L);
   if (n_cols == 0) return VS_OK;
@@ -527,58 +555,49 @@ int eval_at_points(const uint32_t* const* h_cols, uint32_t n_cols, uint32_t L, c
   }
   const uint32_t hb = std::min<uint32_t>(L, EV_LOG_SEG);
   const uint32_t lo_n = 1u << hb, hi_n = 1u << (L - hb), per = lo_n + hi_n;
-  const uint32_t gx = std::max<uint32_t>(
-      1, std::min<uint32_t>((hi_n + EV_UNROLL - 1) / EV_UNROLL, (uint32_t)sm_count() * 4 / n_cols));
-  Scratch s(st);
   qm31* tables = nullptr;
-  uint32_t* partials = nullptr;
   const uint32_t** d_cols = nullptr;
   VS_TRY(s.alloc(&tables, (uint64_t)np * per));
-  VS_TRY(s.alloc(&partials, (uint64_t)n_cols * gx * np * 4));
-  std::vector<const uint32_t*> cols(h_cols, h_cols + n_cols);
-  VS_TRY(s.upload(&d_cols, cols.data(), n_cols));
+  VS_TRY(s.upload(&d_cols, h_cols, n_cols));
   basis_table_kernel<<<blocks_for((uint64_t)np * per, 256), 256, 0, st>>>(mp, np, hb, lo_n, hi_n, tables);
   VS_LAUNCHED("basis_table_kernel");
-  const dim3 grid(gx, n_cols);
+  const dim3 grid(e.gx, n_cols);
   bool ring = hb == EV_LOG_SEG && hi_n >= 4;
   for (uint32_t c = 0; c < n_cols; c++) ring = ring && (reinterpret_cast<uintptr_t>(h_cols[c]) & 15) == 0;
   if (ring) {
-    if (np == 1) eval_points_ring_kernel<1><<<grid, EV_THREADS, 0, st>>>(d_cols, lo_n, hi_n, tables, partials);
-    else eval_points_ring_kernel<2><<<grid, EV_THREADS, 0, st>>>(d_cols, lo_n, hi_n, tables, partials);
+    if (np == 1) eval_points_ring_kernel<1><<<grid, EV_THREADS, 0, st>>>(d_cols, lo_n, hi_n, tables, e.d);
+    else eval_points_ring_kernel<2><<<grid, EV_THREADS, 0, st>>>(d_cols, lo_n, hi_n, tables, e.d);
     VS_LAUNCHED("eval_points_ring_kernel");
   } else {
-    if (np == 1) eval_points_kernel<1><<<grid, EV_THREADS, 0, st>>>(d_cols, hb, lo_n, hi_n, tables, partials);
-    else eval_points_kernel<2><<<grid, EV_THREADS, 0, st>>>(d_cols, hb, lo_n, hi_n, tables, partials);
+    if (np == 1) eval_points_kernel<1><<<grid, EV_THREADS, 0, st>>>(d_cols, hb, lo_n, hi_n, tables, e.d);
+    else eval_points_kernel<2><<<grid, EV_THREADS, 0, st>>>(d_cols, hb, lo_n, hi_n, tables, e.d);
     VS_LAUNCHED("eval_points_kernel");
   }
-  std::vector<uint32_t> hp((uint64_t)n_cols * gx * np * 4);
-  VS_CUDA(cudaMemcpyAsync(hp.data(), partials, hp.size() * 4, cudaMemcpyDeviceToHost, st));
+  return VS_OK;
+}
+// out[c * np + p] = column c at point p; synchronises st.
+int eval_at_points(const uint32_t* const* h_cols, uint32_t n_cols, uint32_t L, const h::Q (*pts)[2], uint32_t np,
+                   h::Q* out, cudaStream_t st) {
+  Scratch s(st);
+  EvPartials e = ev_shape(n_cols, L, np);
+  VS_TRY(s.alloc(&e.d, e.words()));
+  VS_TRY(eval_enqueue(h_cols, L, pts, e, s));
+  if (n_cols == 0) return VS_OK;
+  std::vector<uint32_t> hp(e.words());
+  VS_CUDA(cudaMemcpyAsync(hp.data(), e.d, hp.size() * 4, cudaMemcpyDeviceToHost, st));
   VS_CUDA(cudaStreamSynchronize(st));
-  for (uint32_t c = 0; c < n_cols; c++)
-    for (uint32_t p = 0; p < np; p++) {
-      h::Q acc{{0, 0, 0, 0}};
-      for (uint32_t b = 0; b < gx; b++) {
-        const uint32_t* v = &hp[(((uint64_t)c * gx + b) * np + p) * 4];
-        acc = h::qadd(acc, h::Q{{v[0], v[1], v[2], v[3]}});
-      }
-      out[c * np + p] = acc;
-    }
+  e.sum(hp.data(), out);
   return VS_OK;
 }
 
-// 1024-leaf tile roots of a commitment, through 2^split subtree roots per tile
-// (merkle_tile_split) for trees of 2^20+ leaves; stream-ordered subroot scratch.
+// 1024-leaf tile roots of a commitment (merkle_tile_roots_split); stream-ordered scratch.
 template <class Leaf>
 int tile_roots_split(const Leaf& leaf, uint64_t N, uint32_t* tiles, cudaStream_t st) {
-  const uint32_t sp = merkle_tile_split(N);
-  if (!sp) return merkle_tile_roots(leaf, N, MK_MAX_TL, tiles, st);
-  const uint64_t t = N >> MK_MAX_TL;
-  uint32_t *a = nullptr, *b = nullptr;
-  VS_CUDA(cudaMallocAsync((void**)&a, (t << sp) * 32, st));
-  int rc = check_cuda(cudaMallocAsync((void**)&b, (t << (sp - 1)) * 32, st), "subroot scratch");
-  if (rc == VS_OK) rc = merkle_tile_roots_split(leaf, N, MK_MAX_TL, sp, tiles, a, b, st);
-  cudaFreeAsync(a, st);
-  if (b) cudaFreeAsync(b, st);
+  const uint32_t sp = merkle_tile_split(N, MK_MAX_SPLIT);
+  uint32_t* sub = nullptr;
+  if (sp) VS_CUDA(cudaMallocAsync((void**)&sub, merkle_tile_scratch_bytes(N, sp), st));
+  const int rc = merkle_tile_roots_split(leaf, N, MK_MAX_TL, sp, tiles, sub, st);
+  if (sub) cudaFreeAsync(sub, st);
   return rc;
 }
 
@@ -604,16 +623,9 @@ extern "C" int vs_commit_group_cairo(const uint32_t* d_cols_hc, uint64_t col_str
   uint32_t* cn = nullptr;
   VS_CUDA(cudaMallocAsync((void**)&cn, n_cols * n * 4, st));
   int rc = launch_permute(true, const_cast<uint32_t*>(d_cols_hc), col_stride, cn, n, n_cols, log_n, nullptr, nullptr, st);
-  // 2. stwo coefficients (the reference keeps them for the OODS evaluation)
-  if (rc == VS_OK && d_coeffs) {
-    rc = check_cuda(cudaMemcpyAsync(d_coeffs, cn, n_cols * n * 4, cudaMemcpyDeviceToDevice, st), "coeffs copy");
-    NttTw ti;
-    if (rc == VS_OK) rc = tw_for(TW_STWO, log_n, false, &ti, st);
-    NttColumns io{d_coeffs, d_coeffs, nullptr, nullptr, n, n, n_cols};
-    if (rc == VS_OK) rc = ntt_transform(io, log_n, ti, false, st);
-  }
-  // 3. LDE x4 on the canonic coset, BRT output
-  if (rc == VS_OK) rc = lde_cached(TW_STWO, cn, n, d_eval_cn, N, n_cols, log_n, 2, st);
+  // 2-3. LDE x4 on the canonic coset, BRT output, and the stwo coefficients on the way (the
+  // reference keeps them for the OODS evaluation)
+  if (rc == VS_OK) rc = lde_cached(TW_STWO, cn, n, d_eval_cn, N, n_cols, log_n, 2, st, d_coeffs, n);
   cudaFreeAsync(cn, st);
   // 4-5. ZK blinding (column c += r_c * Z_H) and the half-coset natural copy
   // that the reference's constraint kernels read, fused into one pass when both
@@ -717,6 +729,18 @@ std::vector<h::Q> line_coeffs_from_evals(std::vector<h::Q> e) {
   brev_all(e);
   return e;
 }
+// Whether n columns of at least N words start at one positive stride (16-byte aligned
+// columns then take no copies on their way into a transform).
+bool even_stride(const uint32_t* const* cols, uint32_t n, uint64_t N, uint64_t* stride) {
+  *stride = N;
+  if (n < 2) return true;
+  if (cols[1] < cols[0]) return false;
+  *stride = cols[1] - cols[0];
+  bool even = *stride >= N;
+  for (uint32_t j = 2; j < n; j++) even = even && cols[j] == cols[0] + j * *stride;
+  if (!even) *stride = N;
+  return even;
+}
 void put_q(uint32_t* dst, const h::Q& q) { std::memcpy(dst, q.v, 16); }
 }  // namespace
 
@@ -747,13 +771,17 @@ extern "C" int vs_cairo_oods_fri(void* channel, vs_cairo_oods_fri_io* io, vs_str
   h::Hash root;
 
   // AIR quotient: half-coset natural -> BRT-canonic, SoA4 commitment (prover.rs:1937-1971)
-  uint32_t* qcn[4];
+  uint32_t *qcn[4], *qcn_own = nullptr;
   for (int k = 0; k < 4; k++) {
     qcn[k] = io->quotient_cn[k];
-    if (!qcn[k]) VS_TRY(s.alloc(&qcn[k], N));
-    VS_TRY(launch_permute(true, const_cast<uint32_t*>(io->quotient_hc[k]), N, qcn[k], N, 1, log_eval, nullptr, nullptr,
-                          st));
+    if (!qcn[k] && !qcn_own) VS_TRY(s.alloc(&qcn_own, 4 * N));
+    if (!qcn[k]) qcn[k] = qcn_own + k * N;
   }
+  uint64_t hc_stride = 0, cn_stride = 0;  // limbs at one stride move in one launch
+  const bool hc_even = even_stride(io->quotient_hc, 4, N, &hc_stride), cn_even = even_stride(qcn, 4, N, &cn_stride);
+  for (uint32_t k = 0; k < 4; k += hc_even && cn_even ? 4 : 1)
+    VS_TRY(launch_permute(true, const_cast<uint32_t*>(io->quotient_hc[k]), hc_stride, qcn[k], cn_stride,
+                          hc_even && cn_even ? 4 : 1, log_eval, nullptr, nullptr, st));
   uint32_t* qtiles = io->quotient_tile_roots;
   if (!qtiles) VS_TRY(s.alloc(&qtiles, n_tiles * 8));
   VS_TRY(commit_soa4_tiles(qcn, N, d_root, qtiles, st));
@@ -773,36 +801,62 @@ extern "C" int vs_cairo_oods_fri(void* channel, vs_cairo_oods_fri_io* io, vs_str
   for (uint32_t i = 1; i < log_n; i++) { zh_z = pi_x(zh_z); zh_n = pi_x(zh_n); }
   const h::Q pts[2][2] = {{zx, zy}, {nx, ny}};
 
-  // trace columns at z and z_next from their coefficients, plus r * Z_H (prover.rs:1987-2001)
+  // Sampled values: trace columns at z and z_next from their coefficients
+  // (prover.rs:1987-2001), interaction columns from the first 2^log_n stwo coefficients
+  // of their evaluations (:2037-2048), quotient limbs at z from all their coefficients
+  // (:2053-2065). All partial sums are read back at once.
   std::vector<h::Q> tv(2 * nt), iv(2 * ni);
-  VS_TRY(eval_at_points(io->trace_coeffs, nt, log_n, pts, 2, tv.data(), st));
-  if (io->zk_scalars)
+  h::Q qv[4];
+  NttTw ti;
+  VS_TRY(tw_for(TW_STWO, log_eval, false, &ti, st));
+  const uint32_t B = std::min<uint32_t>(std::max<uint32_t>(ni, 4), 8);
+  std::vector<EvPartials> ev{ev_shape(nt, log_n, 2)};
+  for (uint32_t c0 = 0; c0 < ni; c0 += B) ev.push_back(ev_shape(std::min(B, ni - c0), log_n, 2));
+  ev.push_back(ev_shape(4, log_eval, 1));
+  uint64_t ev_words = 0;
+  for (const EvPartials& e : ev) ev_words += e.words();
+  uint32_t *coef = nullptr, *partials = nullptr;
+  VS_TRY(s.alloc(&coef, B * N));
+  VS_TRY(s.alloc(&partials, ev_words));
+  uint64_t ev_at = 0;
+  for (EvPartials& e : ev) { e.d = partials + ev_at; ev_at += e.words(); }
+  VS_TRY(eval_enqueue(io->trace_coeffs, log_n, pts, ev[0], s));
+  // coefficients of nb columns into coef: straight from columns at one stride, else from copies
+  auto interpolate = [&](const uint32_t* const* cols, uint32_t nb) -> int {
+    uint64_t stride = N;
+    const bool even = even_stride(cols, nb, N, &stride);
+    for (uint32_t j = 0; !even && j < nb; j++)
+      VS_CUDA(cudaMemcpyAsync(coef + j * N, cols[j], N * 4, cudaMemcpyDeviceToDevice, st));
+    return ntt_transform(NttColumns{even ? cols[0] : coef, coef, nullptr, nullptr, even ? stride : N, N, nb}, log_eval,
+                         ti, false, st);
+  };
+  std::vector<const uint32_t*> cp(B);
+  for (uint32_t j = 0; j < B; j++) cp[j] = coef + j * N;
+  for (uint32_t c0 = 0, i = 1; c0 < ni; c0 += B, i++) {
+    const uint32_t nb = std::min(B, ni - c0);
+    VS_TRY(interpolate(io->interaction_evals + c0, nb));
+    VS_TRY(eval_enqueue(cp.data(), log_n, pts, ev[i], s));
+  }
+  VS_TRY(interpolate(qcn, 4));
+  VS_TRY(eval_enqueue(cp.data(), log_eval, pts, ev.back(), s));
+  {
+    std::vector<uint32_t> hp(ev_words);
+    VS_CUDA(cudaMemcpyAsync(hp.data(), partials, ev_words * 4, cudaMemcpyDeviceToHost, st));
+    VS_CUDA(cudaStreamSynchronize(st));
+    const uint32_t* at = hp.data();
+    ev[0].sum(at, tv.data());
+    for (size_t i = 0; i + 1 < ev.size(); i++) {
+      if (i) ev[i].sum(at, iv.data() + 2 * B * (i - 1));
+      at += ev[i].words();
+    }
+    ev.back().sum(at, qv);
+  }
+  if (io->zk_scalars)  // plus r * Z_H of the blinded columns
     for (uint32_t c = 0; c < nt; c++)
       if (const uint32_t r = io->zk_scalars[c]) {
         tv[2 * c] = h::qadd(tv[2 * c], h::qscale(zh_z, r));
         tv[2 * c + 1] = h::qadd(tv[2 * c + 1], h::qscale(zh_n, r));
       }
-  // interaction columns: first 2^log_n stwo coefficients of their evaluations (prover.rs:2037-2048)
-  NttTw ti;
-  VS_TRY(tw_for(TW_STWO, log_eval, false, &ti, st));
-  const uint32_t B = std::min<uint32_t>(std::max<uint32_t>(ni, 4), 8);
-  uint32_t* coef = nullptr;
-  VS_TRY(s.alloc(&coef, B * N));
-  std::vector<const uint32_t*> cp(B);
-  for (uint32_t j = 0; j < B; j++) cp[j] = coef + j * N;
-  for (uint32_t c0 = 0; c0 < ni; c0 += B) {
-    const uint32_t nb = std::min(B, ni - c0);
-    for (uint32_t j = 0; j < nb; j++)
-      VS_CUDA(cudaMemcpyAsync(coef + j * N, io->interaction_evals[c0 + j], N * 4, cudaMemcpyDeviceToDevice, st));
-    VS_TRY(ntt_transform(NttColumns{coef, coef, nullptr, nullptr, N, N, nb}, log_eval, ti, false, st));
-    VS_TRY(eval_at_points(cp.data(), nb, log_n, pts, 2, iv.data() + 2 * c0, st));
-  }
-  // quotient limbs at z from all their coefficients (prover.rs:2053-2065)
-  h::Q qv[4];
-  for (int k = 0; k < 4; k++)
-    VS_CUDA(cudaMemcpyAsync(coef + k * N, qcn[k], N * 4, cudaMemcpyDeviceToDevice, st));
-  VS_TRY(ntt_transform(NttColumns{coef, coef, nullptr, nullptr, N, N, 4}, log_eval, ti, false, st));
-  VS_TRY(eval_at_points(cp.data(), 4, log_eval, pts, 1, qv, st));
 
   // sampled values in flatten_cols order, then the OODS alpha (prover.rs:2067-2095)
   {
@@ -818,8 +872,10 @@ extern "C" int vs_cairo_oods_fri(void* channel, vs_cairo_oods_fri_io* io, vs_str
   // alpha-weighted line coefficients (prover.rs:2095-2150; oods.rs compute_line_coeffs)
   std::vector<uint32_t> bz, cz, bn, cn;
   h::Q lin_z{{0, 0, 0, 0}}, lin_n{{0, 0, 0, 0}}, ap = one;
-  auto push = [&](const h::Q& py, const h::Q& v, std::vector<uint32_t>& bv, std::vector<uint32_t>& cv, h::Q& lin) {
-    const h::Q b = h::qmul(h::qsub(v, h::qconj(v)), h::qinv(h::qsub(py, h::qconj(py))));
+  const h::Q inv_z = h::qinv(h::qsub(zy, h::qconj(zy))), inv_n = h::qinv(h::qsub(ny, h::qconj(ny)));
+  auto push = [&](const h::Q& py, const h::Q& py_inv, const h::Q& v, std::vector<uint32_t>& bv,
+                  std::vector<uint32_t>& cv, h::Q& lin) {
+    const h::Q b = h::qmul(h::qsub(v, h::qconj(v)), py_inv);
     const h::Q a = h::qsub(v, h::qmul(b, py));
     const h::Q wa = h::qmul(ap, a);
     bv.insert(bv.end(), wa.v, wa.v + 4);
@@ -827,11 +883,11 @@ extern "C" int vs_cairo_oods_fri(void* channel, vs_cairo_oods_fri_io* io, vs_str
     lin = h::qadd(lin, h::qmul(ap, b));
     ap = h::qmul(ap, alpha);
   };
-  for (uint32_t c = 0; c < nt; c++) push(zy, tv[2 * c], bz, cz, lin_z);
-  for (int k = 0; k < 4; k++) push(zy, qv[k], bz, cz, lin_z);
-  for (uint32_t c = 0; c < ni; c++) push(zy, iv[2 * c], bz, cz, lin_z);
-  for (uint32_t c = 0; c < nt; c++) push(ny, tv[2 * c + 1], bn, cn, lin_n);
-  for (uint32_t c = 0; c < ni; c++) push(ny, iv[2 * c + 1], bn, cn, lin_n);
+  for (uint32_t c = 0; c < nt; c++) push(zy, inv_z, tv[2 * c], bz, cz, lin_z);
+  for (int k = 0; k < 4; k++) push(zy, inv_z, qv[k], bz, cz, lin_z);
+  for (uint32_t c = 0; c < ni; c++) push(zy, inv_z, iv[2 * c], bz, cz, lin_z);
+  for (uint32_t c = 0; c < nt; c++) push(ny, inv_n, tv[2 * c + 1], bn, cn, lin_n);
+  for (uint32_t c = 0; c < ni; c++) push(ny, inv_n, iv[2 * c + 1], bn, cn, lin_n);
 
   // DEEP numerators over [trace, quotient, interaction] (prover.rs:2152-2207)
   const uint32_t n_all = nt + 4 + ni;
@@ -913,49 +969,85 @@ extern "C" int vs_cairo_oods_fri(void* channel, vs_cairo_oods_fri_io* io, vs_str
   }
   VS_TRY(launch_quotients_combine(d_meta, d_meta + 8, d_meta + 16, d_np, d_np + 2, d_np + 4, d_np + 6, d_meta + 24, 2,
                                   xs, ys, log_eval, (uint32_t)N, oq, st));
+  // From here on the transcript runs on the device, so no layer waits for the host: the
+  // DEEP quotient's commitment (1024-leaf tile roots), then FRI: circle fold with 1/y of
+  // the canonic points and committed line folds down to 8 values, each fold fused with
+  // the commitment of its output (prover.rs:2321-2381). One upload, one read-back.
+  struct Transcript {
+    ChanDev ch;
+    uint32_t roots[33 * 8], alphas[32 * 4];  // DEEP quotient, then FRI layers
+  };
+  auto tr = std::make_unique<Transcript>();
+  std::memcpy(tr->ch.state, ch->state.data(), 32);
+  tr->ch.n_draws = ch->n_draws;
+  tr->ch.error = 0;
+  Transcript* d_tr = nullptr;
+  VS_TRY(s.upload(&d_tr, tr.get(), 1));
+  // layer l folds to 2^(log_eval-1-l) values with challenge l; its step draws challenge l + 1
+  const uint32_t nf = log_eval - 3;
+  auto after = [&](uint32_t root) {  // root 0: the DEEP quotient's
+    return ChannelStep{&d_tr->ch, 0, d_tr->roots, 0, 8 * root, d_tr->alphas, 0, (int)(4 * root)};
+  };
+  const uint32_t* tws[TAIL_MAXF];
+  for (uint32_t l = 0; l < nf; l++)
+    VS_TRY(get_fold_twiddles(l == 0 ? (int)FOLD_CANONIC_CIRCLE : (int)COSET_HALF_ODDS, log_eval - l, &tws[l], st));
   uint32_t* otiles = io->oods_tile_roots;
   if (!otiles) VS_TRY(s.alloc(&otiles, n_tiles * 8));
-  VS_TRY(commit_soa4_tiles(oq, N, d_root, otiles, st));
-  VS_TRY(read_hash(d_root, root, st));
-  std::memcpy(io->oods_root, root.data(), 32);
-  ch->mix_digest(root);
-
-  // FRI: circle fold with 1/y of the canonic points, then committed line folds
-  // down to 8 values; each fold is fused with the commitment of its output
-  // (prover.rs:2321-2381)
-  uint32_t *fri = nullptr, *mscratch = nullptr;
-  VS_TRY(s.alloc(&fri, 4 * N));
-  VS_TRY(s.alloc(&mscratch, merkle_scratch_words_any(N / 2)));
-  const uint32_t split = std::min<uint32_t>(merkle_root_split(log_eval), 5);
-  uint32_t* src[4] = {oq[0], oq[1], oq[2], oq[3]};
-  uint32_t* dst[4];
-  uint64_t off = 0;
-  h::Q fa = ch->draw_felt();
-  std::vector<h::Q> alphas{fa};
-  std::vector<h::Hash> roots;
-  const uint32_t* tw = nullptr;
-  VS_TRY(get_fold_twiddles(FOLD_CANONIC_CIRCLE, log_eval, &tw, st));
-  uint64_t half = N / 2;
-  for (int k = 0; k < 4; k++) dst[k] = fri + off + k * half;
-  off += 4 * half;
-  VS_TRY(fold_commit_layer(src, dst, tw, fa.v, nullptr, false, half, d_root, mscratch, st, split));
-  for (uint32_t cur = log_eval - 1; cur > 3; cur--) {
-    VS_TRY(read_hash(d_root, root, st));
-    ch->mix_digest(root);
-    roots.push_back(root);
-    fa = ch->draw_felt();
-    alphas.push_back(fa);
-    VS_TRY(get_fold_twiddles(COSET_HALF_ODDS, cur, &tw, st));
-    for (int k = 0; k < 4; k++) src[k] = dst[k];
-    half >>= 1;
-    for (int k = 0; k < 4; k++) dst[k] = fri + off + k * half;
-    off += 4 * half;
-    VS_TRY(fold_commit_layer(src, dst, tw, fa.v, nullptr, false, half, d_root, mscratch, st, split));
+  auto tree = [&](uint32_t m, TreeLevels* t) {  // levels kept only to be taken up by the next launch
+    *t = TreeLevels{nullptr, 1, m >= MK_WIDE ? 5u : channel_leaf_tile(m, m), m};
+    return s.alloc(&t->base, TreeLevels::bytes(1, t->s, m) / 4);
+  };
+  const LeafSoa4 oleaf{oq[0], oq[1], oq[2], oq[3]};
+  TreeLevels lv{};
+  VS_TRY(tree(log_eval, &lv));
+  if (N <= 1024) {
+    VS_TRY(commit_with_channel(oleaf, lv, 1, after(0), st));
+    VS_CUDA(cudaMemcpyAsync(otiles, d_tr->roots, 32, cudaMemcpyDeviceToDevice, st));
+  } else {
+    VS_TRY(tile_roots_split(oleaf, N, otiles, st));
+    const uint32_t TL = std::min<uint32_t>(MK_MAX_TL, log_eval - MK_MAX_TL);
+    lv.s = MK_MAX_TL;
+    VS_TRY(channel_tiles(LeafHashes{otiles}, lv, MK_MAX_TL, TL, 1, after(0), st));
+    VS_TRY(channel_levels(lv, MK_MAX_TL + TL, 1, after(0), st));
   }
+  uint32_t* fri = nullptr;
+  VS_TRY(s.alloc(&fri, 4 * N));
+  FriTail tail{};
+  tail.first = nf;
+  Soa4Ptrs src{{oq[0], oq[1], oq[2], oq[3]}};
+  uint32_t* base = fri;
+  for (uint32_t l = 0; l < nf; l++) {
+    const uint32_t m = log_eval - 1 - l;
+    Soa4Out dst;
+    for (int k = 0; k < 4; k++) tail.fri[l][k] = dst.c[k] = base + ((uint64_t)k << m);
+    base += 4ull << m;
+    tail.tw[l] = tws[l];
+    tail.tree[l] = TreeLevels{nullptr, 1, 32, m};  // no level is kept (32 is above every level)
+    if (m > TAIL_LOG) {
+      VS_TRY(tree(m, &lv));
+      VS_TRY(commit_with_channel(LeafFoldAt{src, dst, tws[l], d_tr->alphas + 4 * l}, lv, 1, after(1 + l), st));
+      for (int k = 0; k < 4; k++) src.c[k] = dst.c[k];
+    } else if (l < tail.first) {
+      tail.first = l;
+      tail.step = after(1 + l);
+      for (int k = 0; k < 4; k++) tail.in[k] = src.c[k];
+    }
+  }
+  tail.nf = nf;
+  tail.log_eval = log_eval;
+  VS_TRY(launch_fri_tail<false>(tail, 1, st));
   std::vector<uint32_t> planes(32);
-  for (int k = 0; k < 4; k++)
-    VS_CUDA(cudaMemcpyAsync(planes.data() + 8 * k, dst[k], 32, cudaMemcpyDeviceToHost, st));
+  VS_CUDA(cudaMemcpyAsync(planes.data(), tail.fri[nf - 1][0], 128, cudaMemcpyDeviceToHost, st));
+  VS_CUDA(cudaMemcpyAsync(tr.get(), d_tr, sizeof(Transcript), cudaMemcpyDeviceToHost, st));
   VS_CUDA(cudaStreamSynchronize(st));
+  if (tr->ch.error) return set_error(VS_ERR_CUDA, "vs_cairo_oods_fri: no challenge drawn in 64 squeezes");
+  std::memcpy(ch->state.data(), tr->ch.state, 32);
+  ch->n_draws = tr->ch.n_draws;
+  std::memcpy(io->oods_root, tr->roots, 32);
+  std::vector<h::Q> alphas(nf);
+  for (uint32_t l = 0; l < nf; l++) std::memcpy(alphas[l].v, tr->alphas + 4 * l, 16);
+  std::vector<h::Hash> roots(nf - 1);
+  for (uint32_t l = 0; l + 1 < nf; l++) std::memcpy(roots[l].data(), tr->roots + 8 * (1 + l), 32);
   std::vector<h::Q> last(8);
   for (int i = 0; i < 8; i++) last[i] = h::Q{{planes[i], planes[8 + i], planes[16 + i], planes[24 + i]}};
   const std::vector<h::Q> nat = line_coeffs_from_evals(last);

@@ -6,7 +6,6 @@
 // is never re-read for its commitment.
 #include <algorithm>
 
-#include "fri.h"
 #include "fri_impl.cuh"
 #include "merkle.h"
 #include "twiddles.h"
@@ -76,19 +75,6 @@ __global__ void __launch_bounds__(256) fold_chain_kernel(FoldChain p) {
     }
     __syncthreads();
   }
-}
-
-// One fold layer + its Merkle root. src/dst are SoA4 plane pointers; `half_n`
-// = output size (power of two); twiddles of length half_n.
-int fold_commit_layer(const uint32_t* const src[4], uint32_t* const dst[4], const uint32_t* tw, const uint32_t* alpha,
-                      const uint32_t* alpha_sq, bool circle_accumulate, uint64_t half_n, uint32_t* d_root,
-                      uint32_t* scratch, cudaStream_t st, uint32_t split) {
-  LeafFold leaf{};
-  for (int k = 0; k < 4; k++) { leaf.src.c[k] = src[k]; leaf.dst.c[k] = dst[k]; }
-  leaf.tw = tw;
-  for (int k = 0; k < 4; k++) { leaf.alpha.v[k] = alpha[k]; leaf.alpha_sq.v[k] = alpha_sq ? alpha_sq[k] : 0; }
-  leaf.accumulate = circle_accumulate ? 1 : 0;
-  return merkle_root(leaf, half_n, d_root, st, scratch, split);
 }
 
 }  // namespace vs

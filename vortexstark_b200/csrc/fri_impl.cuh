@@ -56,4 +56,16 @@ struct LeafFold {
   }
 };
 
+// The same leaf without accumulation, its challenge (4 words) in device memory.
+struct LeafFoldAt {
+  Soa4Ptrs src;
+  Soa4Out dst;
+  const uint32_t* tw;
+  const uint32_t* alpha;
+  __device__ __forceinline__ void operator()(uint64_t i, uint32_t out[8]) const {
+    LeafFold f{src, dst, tw, qm31{{__ldg(alpha), __ldg(alpha + 1), __ldg(alpha + 2), __ldg(alpha + 3)}}, qzero(), 0};
+    f(i, out);
+  }
+};
+
 }  // namespace vs

@@ -26,7 +26,7 @@ constexpr int MK_MAX_TL = 10;
 inline unsigned merkle_smem_bytes(uint32_t TL) { return (8u << TL) * 4u + (TL ? (8u << (TL - 1)) * 4u : 0u); }
 
 // The kept levels of `jobs` equal trees of 2^m leaves each: level k (s <= k <= m) is
-// [jobs][2^(m-k)] hashes of 8 words, one level after the other.
+// [jobs][2^(m-k)] hashes of 8 words, one level after the other (s > m: none is kept).
 struct TreeLevels {
   uint32_t* base;
   uint32_t jobs, s, m;

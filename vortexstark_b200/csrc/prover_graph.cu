@@ -295,7 +295,7 @@ struct GraphProver::Impl {
   TreeBufs trace_t, quot_t;
   std::vector<TreeBufs> fri_t;
   // subroot scratch shared by the trees (committed one after another in the graph)
-  uint32_t split = 0, *sub_a = nullptr, *sub_b = nullptr;
+  uint32_t split = 0, *sub = nullptr;
   ArenaLayout lay;
   cudaGraphExec_t exec = nullptr;
   cudaGraph_t graph = nullptr;
@@ -337,7 +337,7 @@ struct GraphProver::Impl {
   template <class Leaf>
   int commit(const Leaf& leaf, TreeBufs& t) {
     const uint32_t sp = (t.TL == MK_MAX_TL && t.n >= (1ull << 20)) ? split : 0u;
-    VS_TRY(merkle_tile_roots_split(leaf, t.n, t.TL, sp, t.layers[0], sub_a, sub_b, st));
+    VS_TRY(merkle_tile_roots_split(leaf, t.n, t.TL, sp, t.layers[0], sub, st));
     for (size_t k = 1; k < t.layers.size(); k++)
       VS_TRY(launch_hash_nodes(t.layers[k - 1], t.layers[k], t.n >> (t.TL + k), st));
     return VS_OK;
@@ -375,10 +375,7 @@ struct GraphProver::Impl {
     VS_TRY(tree_bufs(trace_t, N));
     VS_TRY(tree_bufs(quot_t, N));
     split = merkle_tile_split(N);  // fixed for the prover's lifetime (its graph is captured once)
-    if (split) {
-      VS_TRY(alloc(&sub_a, ((N >> MK_MAX_TL) << split) * 8));
-      VS_TRY(alloc(&sub_b, ((N >> MK_MAX_TL) << (split - 1)) * 8));
-    }
+    if (split) VS_TRY(alloc(&sub, merkle_tile_scratch_bytes(N, split) / 4));
     fri_t.resize(nf);
     for (uint32_t l = 0; l < nf; l++) {
       const uint64_t half = N >> (l + 1);
