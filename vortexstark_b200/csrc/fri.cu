@@ -13,9 +13,10 @@
 
 namespace vs {
 
-// FRI layers of at most 2^FRI_FOREST_LOG values take the shared launches of
-// vs_fri_fold_commit.
-constexpr uint32_t FRI_FOREST_LOG = 20;
+// FRI layers of at most 2^fri_forest_log values take the shared launches of
+// vs_fri_fold_commit. Measured (us, layers from 2^19 / 2^20 / 2^21 down): chains of 2^21
+// 251 / 244 / 244, of 2^22 435 / 445 / 466, of 2^24 1496 / 1506 / 1524.
+inline uint32_t fri_forest_log(uint32_t log_n) { return log_n <= 21 ? 20 : 19; }
 
 __global__ void fold_line_kernel(Soa4Ptrs in, const uint32_t* __restrict__ tw, Soa4Out out, qm31 alpha,
                                  uint32_t half_n) {
@@ -53,7 +54,17 @@ struct FoldChain {
 };
 __global__ void __launch_bounds__(256) fold_chain_kernel(FoldChain p) {
   __shared__ __align__(8) uint32_t sm[2][4][1 << (FOLD_CHAIN - 1)];
+  // a thread's first twiddle of a layer, fetched a layer ahead
+  uint32_t tw_next = 0;
+  auto fetch_tw = [&](uint32_t l) {
+    if (l >= p.n) return;
+    const uint32_t cnt = 1u << (p.c - 1 - l);
+    if (threadIdx.x < cnt) tw_next = __ldg(p.tw[l] + (uint64_t)blockIdx.x * cnt + threadIdx.x);
+  };
+  fetch_tw(0);
   for (uint32_t l = 0; l < p.n; l++) {
+    const uint32_t tw_first = tw_next;
+    fetch_tw(l + 1);
     const uint32_t cnt = 1u << (p.c - 1 - l);              // this CTA's values of layer l
     const uint64_t base = (uint64_t)blockIdx.x * cnt, size = 1ull << (p.log_in - 1 - l);
     const uint32_t(*in)[1 << (FOLD_CHAIN - 1)] = sm[(l + 1) & 1];
@@ -65,7 +76,7 @@ __global__ void __launch_bounds__(256) fold_chain_kernel(FoldChain p) {
         f0.v[k] = w.x;
         f1.v[k] = w.y;
       }
-      const qm31 r = fold_pair(f0, f1, p.alpha[l], __ldg(p.tw[l] + base + i));
+      const qm31 r = fold_pair(f0, f1, p.alpha[l], i == threadIdx.x ? tw_first : __ldg(p.tw[l] + base + i));
 #pragma unroll
       for (int k = 0; k < 4; k++) {
         sm[l & 1][k][i] = r.v[k];
@@ -116,7 +127,7 @@ int vs_fri_fold_commit(const uint32_t* d_src, uint32_t log_n, const uint32_t* h_
   // first, several to a launch, and their trees share launches, as do the upper
   // levels of all trees. Taken alone, a small layer is two launches that leave the
   // chip idle (about 30 us at any size below 2^17).
-  const uint32_t n_big = log_n - 1 > FRI_FOREST_LOG ? log_n - 1 - FRI_FOREST_LOG : 0;
+  const uint32_t n_big = log_n - 1 > fri_forest_log(log_n) ? log_n - 1 - fri_forest_log(log_n) : 0;
   const uint32_t split = std::min<uint32_t>(merkle_root_split(log_n), 5);
   const uint32_t small_log = log_n - 1 - n_big;  // log2 of the first small layer
   const uint32_t TL = small_log <= 9 ? 9 : std::min<uint32_t>(MK_MAX_TL, std::max<uint32_t>(8, small_log - 8));

@@ -14,6 +14,11 @@ namespace vs {
 // One level of parents: parents[i] = Blake2s(children[2i] || children[2i+1]).
 int launch_hash_nodes(const uint32_t* children, uint32_t* parents, uint64_t n_parents, cudaStream_t st);
 
+// Threads of a tile that is reduced to its root: one a leaf, at most MK_THREADS (the
+// kernels' loops step by MK_THREADS, so a smaller block must cover the tile at once). The
+// 2^10 tiles of 128 hashes behind a 2^20-leaf tile-root tree are then resident together.
+inline unsigned merkle_tile_threads(uint32_t TL) { return std::min<unsigned>(MK_THREADS, std::max<unsigned>(32, 1u << TL)); }
+
 // stop_log (<= TL): 2^stop_log roots per tile instead of one (merkle_subtree_kernel).
 template <class Leaf>
 int merkle_tile_roots(const Leaf& leaf, uint64_t n_leaves, uint32_t TL, uint32_t* roots, cudaStream_t st,
@@ -21,7 +26,8 @@ int merkle_tile_roots(const Leaf& leaf, uint64_t n_leaves, uint32_t TL, uint32_t
   const unsigned smem = merkle_smem_bytes(TL);  // at most 48 KiB (TL <= 10): no opt-in needed
   const uint64_t tiles = (n_leaves + (1ull << TL) - 1) >> TL;
   if (stop_log > TL) stop_log = TL;
-  merkle_subtree_kernel<Leaf><<<(unsigned)tiles, MK_THREADS, smem, st>>>(leaf, TL, n_leaves, roots, stop_log);
+  const unsigned threads = stop_log ? MK_THREADS : merkle_tile_threads(TL);
+  merkle_subtree_kernel<Leaf><<<(unsigned)tiles, threads, smem, st>>>(leaf, TL, n_leaves, roots, stop_log);
   VS_LAUNCHED("merkle_subtree_kernel");
   return VS_OK;
 }

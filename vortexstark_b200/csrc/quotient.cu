@@ -32,6 +32,11 @@ __global__ void zero_pad_kernel(const uint32_t* __restrict__ src, uint32_t* __re
   uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < dst_n) dst[i] = i < src_n ? src[i] : 0u;
 }
+// The same with 16-byte accesses (n4, src4 in 16-byte units; the host checks alignment).
+__global__ void zero_pad4_kernel(const uint4* __restrict__ src, uint4* __restrict__ dst, uint32_t src4, uint32_t n4) {
+  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n4) dst[i] = i < src4 ? src[i] : make_uint4(0u, 0u, 0u, 0u);
+}
 __global__ void interleave_kernel(const uint32_t* __restrict__ e, const uint32_t* __restrict__ o,
                                   uint32_t* __restrict__ out, uint32_t half_n) {
   uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -368,7 +373,12 @@ void cuda_fibonacci_quotient(const uint32_t* trace, uint32_t* o0, uint32_t* o1, 
 }
 void cuda_zero_pad(const uint32_t* src, uint32_t* dst, uint32_t src_n, uint32_t dst_n) {
   if (!dst_n) return;
-  zero_pad_kernel<<<blocks_for(dst_n, 256), 256>>>(src, dst, src_n, dst_n);
+  const bool vec = ((reinterpret_cast<uintptr_t>(src) | reinterpret_cast<uintptr_t>(dst)) & 15) == 0 && src_n % 4 == 0 && dst_n % 4 == 0;
+  if (vec)
+    zero_pad4_kernel<<<blocks_for(dst_n / 4, 256), 256>>>(reinterpret_cast<const uint4*>(src), reinterpret_cast<uint4*>(dst),
+                                                          src_n / 4, dst_n / 4);
+  else
+    zero_pad_kernel<<<blocks_for(dst_n, 256), 256>>>(src, dst, src_n, dst_n);
   check_cuda(cudaGetLastError(), "cuda_zero_pad");
 }
 void cuda_interleave_u32(const uint32_t* even, const uint32_t* odd, uint32_t* out, uint32_t half_n) {

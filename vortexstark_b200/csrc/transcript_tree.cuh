@@ -107,7 +107,15 @@ __global__ void __launch_bounds__(MK_THREADS, 2) fri_tail_kernel(FriTail p) {
   uint32_t* sm = tail_sm + 2 * 4 * (1 << TAIL_LOG);
   const uint32_t j = blockIdx.x;
   ChannelStep step = p.step;
+  // a thread's first twiddle of a layer, fetched a layer ahead (a layer has at most two a thread)
+  uint32_t tw_next = 0;
+  auto fetch_tw = [&](uint32_t l) {
+    if (l < p.nf && threadIdx.x < (1u << (p.log_eval - 1 - l))) tw_next = __ldg(p.tw[l] + threadIdx.x);
+  };
+  fetch_tw(p.first);
   for (uint32_t l = p.first; l < p.nf; l++) {
+    const uint32_t tw_first = tw_next;
+    fetch_tw(l + 1);
     const uint32_t m = p.log_eval - 1 - l, half = 1u << m;
     const volatile uint32_t* al = step.alpha + (uint64_t)j * step.astride + p.alpha0 + 4 * l;
     const qm31 alpha{{al[0], al[1], al[2], al[3]}};
@@ -120,7 +128,7 @@ __global__ void __launch_bounds__(MK_THREADS, 2) fri_tail_kernel(FriTail p) {
         f0.v[k] = x.x;
         f1.v[k] = x.y;
       }
-      const qm31 r = fold_pair(f0, f1, alpha, __ldg(p.tw[l] + i));
+      const qm31 r = fold_pair(f0, f1, alpha, i == threadIdx.x ? tw_first : __ldg(p.tw[l] + i));
 #pragma unroll
       for (int k = 0; k < 4; k++) {
         val[l & 1][k][i] = w[k] = r.v[k];
@@ -180,7 +188,7 @@ int channel_tiles(const Leaf& leaf, const TreeLevels& t, uint32_t k, uint32_t TL
                   cudaStream_t st) {
   // the channel step's 24 words follow the root, wherever the levels left it
   const unsigned smem = std::max(merkle_smem_bytes(TL), (8u << TL) * 4 + 128);
-  channel_tile_kernel<Leaf><<<jobs << (t.m - k - TL), MK_THREADS, smem, st>>>(leaf, t, k, TL, c);
+  channel_tile_kernel<Leaf><<<jobs << (t.m - k - TL), merkle_tile_threads(TL), smem, st>>>(leaf, t, k, TL, c);
   VS_LAUNCHED("channel_tile_kernel");
   return VS_OK;
 }
