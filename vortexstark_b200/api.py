@@ -8,13 +8,13 @@ Tensors are int32 views of u32 field words, on a CUDA device.
 from __future__ import annotations
 
 import ctypes as C
-import threading
 
 import torch
 
 from . import check, lib
 
-PROOF_CAP = 32 << 20  # bytes; the largest proof (log_n = 28) is a few MB
+PROOF_CAP = 32 << 20  # bytes; more than the largest proof (log_n = 28: a few MB)
+
 
 
 def _stream(stream=None) -> int:
@@ -74,23 +74,25 @@ def fri_fold_commit(src: torch.Tensor, log_n: int, alphas, work: torch.Tensor, r
           "vs_fri_fold_commit")
 
 
-_tls = threading.local()
+_new_bytes_fn = C.PYFUNCTYPE(C.py_object, C.c_void_p, C.c_ssize_t)(("PyBytes_FromStringAndSize", C.pythonapi))
+_bytes_addr = C.PYFUNCTYPE(C.c_void_p, C.py_object)(("PyBytes_AsString", C.pythonapi))
 
 
-def _proof_buffer():
-    """One reusable host buffer per thread for proofs coming back from the library."""
-    buf = getattr(_tls, "buf", None)
-    if buf is None:
-        buf = _tls.buf = (C.c_uint8 * PROOF_CAP)()
-    return buf
+def _result_bytes(n: int):
+    """An n-byte bytes object that the library fills before anyone sees it, and its address."""
+    b = _new_bytes_fn(None, n)
+    return b, _bytes_addr(b)
 
 
 def prove_fib(a: int, b: int, log_n: int, stream=None) -> bytes:
     """Fibonacci proof in the KRAK v1 wire format."""
-    buf = _proof_buffer()
     n = C.c_uint64(0)
-    check(lib().vs_prove_fib(a, b, log_n, buf, PROOF_CAP, C.byref(n), _stream(stream)), "vs_prove_fib")
-    return C.string_at(buf, n.value)
+    rc = lib().vs_prove_fib(a, b, log_n, None, 0, C.byref(n), _stream(stream))  # the length
+    if n.value == 0:
+        check(rc, "vs_prove_fib")
+    out, ptr = _result_bytes(n.value)
+    check(lib().vs_prove_fib(a, b, log_n, ptr, n.value, C.byref(n), _stream(stream)), "vs_prove_fib")
+    return out
 
 
 def commit_seeded(log_n: int, n_cols: int, seed: int, blowup: int = 2, stream=None) -> bytes:
@@ -227,7 +229,6 @@ class Engine:
         self.h = C.c_void_p()
         flags = 0 if size_priority else 1
         check(lib().vs_engine_create_ex(slots, hbm_budget_bytes, flags, C.byref(self.h)), "vs_engine_create_ex")
-        self._buf = (C.c_uint8 * PROOF_CAP)()
 
     def prepare(self, job: Job) -> None:
         check(lib().vs_engine_prepare(self.h, C.byref(job)), "vs_engine_prepare")
@@ -248,17 +249,26 @@ class Engine:
         """Returns (result bytes, t_submit, t_start, t_end) in engine seconds. With a
         timeout, raises VstarkError (status VS_ERR_TIMEOUT = 5) when the job is not
         done in time; the ticket stays valid."""
+        rc, r, out = self._wait(ticket, timeout_s)
+        check(rc, "vs_engine_wait")
+        return out, r.t_submit, r.t_start, r.t_end
+
+    def _wait(self, ticket: int, timeout_s: float | None):
+        """(status, record, result bytes): the length first, then the bytes straight into the
+        object that is returned; a failed ticket is retired by the second call too."""
         r = JobResult()
         t = -1.0 if timeout_s is None else float(timeout_s)
-        check(lib().vs_engine_wait_for(self.h, ticket, t, C.byref(r), self._buf, PROOF_CAP), "vs_engine_wait")
-        return C.string_at(self._buf, r.out_len), r.t_submit, r.t_start, r.t_end
+        rc = lib().vs_engine_wait_for(self.h, ticket, t, C.byref(r), None, 0)
+        if rc != 0 and r.status == 0:  # not finished, or no such ticket
+            return rc, r, b""
+        out, ptr = _result_bytes(r.out_len)
+        rc = lib().vs_engine_wait_for(self.h, ticket, t, C.byref(r), ptr, r.out_len)
+        return rc, r, out
 
     def wait_status(self, ticket: int, timeout_s: float | None = None) -> tuple[int, bytes]:
         """(status, result bytes) without raising; status 0 = done."""
-        r = JobResult()
-        t = -1.0 if timeout_s is None else float(timeout_s)
-        rc = lib().vs_engine_wait_for(self.h, ticket, t, C.byref(r), self._buf, PROOF_CAP)
-        return rc, (C.string_at(self._buf, r.out_len) if rc == 0 else b"")
+        rc, _, out = self._wait(ticket, timeout_s)
+        return rc, (out if rc == 0 else b"")
 
     def cancel(self, ticket: int) -> int:
         """0 when the queued job was cancelled; VS_ERR_BUSY (7) when it already runs or ran."""

@@ -571,8 +571,10 @@ int vs_engine_wait_for(void* h, uint64_t ticket, double timeout_s, vs_job_result
   }
   if (!out) return VS_OK;  // length query; the result stays available
   if (cap < r.bytes.size()) return set_error(VS_ERR_INVALID, "result needs %zu bytes", r.bytes.size());
-  std::copy(r.bytes.begin(), r.bytes.end(), out);
+  const std::vector<uint8_t> bytes = std::move(r.bytes);
   e->results.erase(it);
+  lk.unlock();  // slots report their jobs while this one's megabyte is copied and freed
+  std::copy(bytes.begin(), bytes.end(), out);
   return VS_OK;
 }
 
