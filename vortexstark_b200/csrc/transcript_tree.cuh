@@ -36,6 +36,35 @@ static __device__ __noinline__ void channel_compress(uint32_t* h, const uint32_t
 #pragma unroll
   for (int i = 0; i < 8; i++) h[i] = hh[i];
 }
+// Mixes `root` into the state in blk[0..8) and, with `draw`, leaves a challenge in h[0..4).
+// Run by one thread on shared memory: root and h 8 words, blk 16. Returns the draws made,
+// 0 when 64 were not enough.
+__device__ __forceinline__ uint32_t channel_mix_draw(uint32_t* blk, uint32_t* h, const uint32_t* root, bool draw) {
+#pragma unroll
+  for (int i = 0; i < 8; i++) blk[8 + i] = root[i];
+  b2s_init(h);
+  channel_compress(h, blk, 64u, true);  // state || digest
+#pragma unroll
+  for (int i = 0; i < 8; i++) blk[i] = h[i];
+  if (!draw) return 0;
+#pragma unroll
+  for (int i = 9; i < 16; i++) blk[i] = 0;
+  for (uint32_t draws = 1; draws <= 64; draws++) {  // until all words are below 2p
+    blk[8] = draws - 1;
+    b2s_init(h);
+    channel_compress(h, blk, 37u, true);  // state || counter || 0x00
+    bool ok = true;
+#pragma unroll
+    for (int i = 0; i < 8; i++) ok = ok && h[i] < 2u * VS_P;
+    if (!ok) continue;
+#pragma unroll
+    for (int i = 0; i < 4; i++) h[i] %= VS_P;
+    return draws;
+  }
+#pragma unroll
+  for (int i = 0; i < 4; i++) h[i] = 0;
+  return 0;
+}
 // Run by one thread; the root (8 words) and 24 words of scratch are in shared memory.
 __device__ __forceinline__ void channel_step(const ChannelStep& s, uint32_t j, const uint32_t* root, uint32_t* scratch) {
   uint32_t *blk = scratch, *h = scratch + 16;
@@ -43,31 +72,17 @@ __device__ __forceinline__ void channel_step(const ChannelStep& s, uint32_t j, c
   uint32_t* ar = s.arena + (uint64_t)j * s.words + s.arena_off;
 #pragma unroll
   for (int i = 0; i < 8; i++) {
-    blk[8 + i] = ar[i] = root[i];
+    ar[i] = root[i];
     blk[i] = s.reset ? 0u : c->state[i];
   }
-  b2s_init(h);
-  channel_compress(h, blk, 64u, true);  // state || digest
+  const bool draw = s.alpha_off >= 0;
+  const uint32_t draws = channel_mix_draw(blk, h, root, draw);
 #pragma unroll
-  for (int i = 0; i < 8; i++) blk[i] = c->state[i] = h[i];
-  uint32_t draws = 0, error = s.reset ? 0u : c->error;
-  if (s.alpha_off >= 0) {
-#pragma unroll
-    for (int i = 9; i < 16; i++) blk[i] = 0;
-    bool ok = false;
-    while (!ok && draws < 64) {  // until all words are below 2p
-      blk[8] = draws++;
-      b2s_init(h);
-      channel_compress(h, blk, 37u, true);  // state || counter || 0x00
-      ok = true;
-#pragma unroll
-      for (int i = 0; i < 8; i++) ok = ok && h[i] < 2u * VS_P;
-    }
-    if (!ok) error = 1;
-    for (int i = 0; i < 4; i++) s.alpha[(uint64_t)j * s.astride + s.alpha_off + i] = ok ? h[i] % VS_P : 0u;
-  }
+  for (int i = 0; i < 8; i++) c->state[i] = blk[i];
+  for (int i = 0; draw && i < 4; i++) s.alpha[(uint64_t)j * s.astride + s.alpha_off + i] = h[i];
   c->n_draws = draws;
-  c->error = error;
+  if (s.reset) c->error = 0;
+  if (draw && !draws) c->error = 1;
 }
 
 // One CTA per tile of 2^TL hashes of tree level k (leaves: k = 0): every kept level
@@ -87,6 +102,7 @@ __global__ void __launch_bounds__(MK_THREADS) channel_tile_kernel(Leaf leaf, Tre
 // Layer l has 2^(log_eval-1-l) values; its challenge is at alpha0 + 4 l of the job's slots.
 constexpr uint32_t TAIL_LOG = 9;
 constexpr int TAIL_MAXF = 28;
+constexpr uint32_t TAIL_TILE_WORDS = 12u << TAIL_LOG;  // merkle_smem_bytes(TAIL_LOG) / 4
 struct FriTail {
   uint32_t first, nf, log_eval;        // layers first (>= 1) .. nf - 1
   uint32_t alpha0;
@@ -105,20 +121,18 @@ __global__ void __launch_bounds__(MK_THREADS, 2) fri_tail_kernel(FriTail p) {
   extern __shared__ __align__(16) uint32_t tail_sm[];
   uint32_t(*val)[4][1 << TAIL_LOG] = reinterpret_cast<uint32_t(*)[4][1 << TAIL_LOG]>(tail_sm);
   uint32_t* sm = tail_sm + 2 * 4 * (1 << TAIL_LOG);
+  uint32_t *blk = sm + TAIL_TILE_WORDS, *h = blk + 48;  // the channel's blocks and digest
   const uint32_t j = blockIdx.x;
-  ChannelStep step = p.step;
-  // a thread's first twiddle of a layer, fetched a layer ahead (a layer has at most two a thread)
-  uint32_t tw_next = 0;
-  auto fetch_tw = [&](uint32_t l) {
-    if (l < p.nf && threadIdx.x < (1u << (p.log_eval - 1 - l))) tw_next = __ldg(p.tw[l] + threadIdx.x);
-  };
-  fetch_tw(p.first);
+  // the channel state stays in shared memory between layers; a layer's challenge is h
+  ChanDev* c = p.step.ch + j;
+  uint32_t* al = p.step.alpha + (uint64_t)j * p.step.astride + p.alpha0;
+  uint32_t* ar = p.step.arena + (uint64_t)j * p.step.words;
+  if (threadIdx.x < 8) blk[threadIdx.x] = c->state[threadIdx.x];
+  if (threadIdx.x < 4) h[threadIdx.x] = al[4 * p.first + threadIdx.x];
+  __syncthreads();
   for (uint32_t l = p.first; l < p.nf; l++) {
-    const uint32_t tw_first = tw_next;
-    fetch_tw(l + 1);
     const uint32_t m = p.log_eval - 1 - l, half = 1u << m;
-    const volatile uint32_t* al = step.alpha + (uint64_t)j * step.astride + p.alpha0 + 4 * l;
-    const qm31 alpha{{al[0], al[1], al[2], al[3]}};
+    const qm31 alpha{{h[0], h[1], h[2], h[3]}};
     auto fold = [&](uint32_t i, uint32_t w[4]) {
       qm31 f0, f1;
 #pragma unroll
@@ -128,7 +142,7 @@ __global__ void __launch_bounds__(MK_THREADS, 2) fri_tail_kernel(FriTail p) {
         f0.v[k] = x.x;
         f1.v[k] = x.y;
       }
-      const qm31 r = fold_pair(f0, f1, alpha, i == threadIdx.x ? tw_first : __ldg(p.tw[l] + i));
+      const qm31 r = fold_pair(f0, f1, alpha, __ldg(p.tw[l] + i));
 #pragma unroll
       for (int k = 0; k < 4; k++) {
         val[l & 1][k][i] = w[k] = r.v[k];
@@ -147,20 +161,22 @@ __global__ void __launch_bounds__(MK_THREADS, 2) fri_tail_kernel(FriTail p) {
           b2s_single(h, w, 4);
         },
         m, 0, half, 1, sm, KeepLevels{p.tree[l], j, m});
-    if (threadIdx.x == 0) channel_step(step, j, root, root + 8);
-    step.arena_off += 8;
-    // layer l + 1's step draws layer l + 2's challenge
-    step.alpha_off = l + 2 < p.nf ? (int)(p.alpha0 + 4 * (l + 2)) : -1;
-    __syncthreads();  // challenge and channel state before the next layer
+    if (threadIdx.x == 0) {  // mix the root; the next layer's challenge
+      const bool draw = l + 1 < p.nf;
+      const uint32_t draws = channel_mix_draw(blk, h, root, draw);
+      for (int i = 0; i < 8; i++) ar[p.step.arena_off + 8 * (l - p.first) + i] = root[i];
+      for (int i = 0; draw && i < 4; i++) al[4 * (l + 1) + i] = h[i];
+      for (int i = 0; i < 8; i++) c->state[i] = blk[i];
+      c->n_draws = draws;
+      if (draw && !draws) c->error = 1;
+    }
+    __syncthreads();  // challenge before the next layer
   }
   // mix_felts(last layer): state || 8 values, 160 bytes
   uint32_t(*v)[1 << TAIL_LOG] = val[(p.nf - 1) & 1];
-  ChanDev* c = step.ch + j;
-  uint32_t* ar = step.arena + (uint64_t)j * step.words;
-  uint32_t *blk = sm, *h = sm + 48;  // 3 blocks of 16 words; the new state
-  if (threadIdx.x < 48) {
+  if (threadIdx.x >= 8 && threadIdx.x < 48) {
     const uint32_t w = threadIdx.x;
-    blk[w] = w < 8 ? c->state[w] : (w < 40 ? v[(w - 8) & 3][(w - 8) >> 2] : 0u);
+    blk[w] = w < 40 ? v[(w - 8) & 3][(w - 8) >> 2] : 0u;
   }
   if (threadIdx.x < 32) ar[p.a_last + threadIdx.x] = v[threadIdx.x & 3][threadIdx.x >> 2];
   __syncthreads();
@@ -175,7 +191,7 @@ __global__ void __launch_bounds__(MK_THREADS, 2) fri_tail_kernel(FriTail p) {
   if (threadIdx.x < N_QUERIES) {
     ChanDev d;
 #pragma unroll
-    for (int i = 0; i < 8; i++) d.state[i] = blk[48 + i];
+    for (int i = 0; i < 8; i++) d.state[i] = h[i];
     d.n_draws = threadIdx.x;
     const uint32_t q = ch_draw_pow2(d, p.log_eval);
     p.qidx[j * N_QUERIES + threadIdx.x] = q;
@@ -226,7 +242,7 @@ int commit_with_channel(const Leaf& leaf, const TreeLevels& t, uint32_t jobs, co
 template <bool QUERIES>
 int launch_fri_tail(FriTail& p, uint32_t jobs, cudaStream_t st) {
   for (int k = 0; k < 4 && !p.in[k]; k++) p.in[k] = p.fri[p.first - 1][k];
-  const unsigned smem = merkle_smem_bytes(TAIL_LOG) + 2 * 4 * (4u << TAIL_LOG);  // 40 KiB: no opt-in needed
+  const unsigned smem = 4 * (TAIL_TILE_WORDS + 2 * 4 * (1u << TAIL_LOG) + 56);  // 40 KiB: no opt-in needed
   fri_tail_kernel<QUERIES><<<jobs, MK_THREADS, smem, st>>>(p);
   VS_LAUNCHED("fri_tail_kernel");
   return VS_OK;
