@@ -57,3 +57,35 @@ def test_small_transforms(log_n):
                                      log_n - 1, 1 << log_n, 2)
     for c, v in zip(cols, (x, x[::-1])):
         assert np.array_equal(host(c), O.native_evaluate(v.copy(), log_n))
+
+
+EDGE = np.array([0, 1, 2**30 - 1, 2**30, 2**30 + 1, 2**31 - 2], dtype=np.uint32)
+
+
+@pytest.mark.parametrize("forward", [True, False])
+def test_butterfly_at_the_ends_of_its_ranges(forward):
+    """One layer over every triple of edge values and twiddles."""
+    v0, v1, t = (a.reshape(-1) for a in np.meshgrid(EDGE, EDGE, EDGE, indexing="ij"))
+    n = 2 * len(t)
+    d, tw = np.zeros(512, np.uint32), np.zeros(256, np.uint32)
+    d[0:n:2], d[1:n:2], tw[:n // 2] = v0, v1, t
+    g = dev(d)
+    V.lib().cuda_circle_ntt_layer(ptr(g), ptr(dev(tw)), 0, 512, int(forward))
+    assert np.array_equal(host(g), O.ntt_layer(d, tw, 0, forward))
+
+
+@pytest.mark.parametrize("log_n", [5, 9, 13, 14, 17, 20, 22])
+def test_edge_values_through_every_pass_form(log_n):
+    """Words at the ends of [0, p) stay in range between layers, rounds and passes."""
+    x = EDGE[np.random.default_rng(log_n).integers(0, len(EDGE), (2, 1 << log_n))]
+    x[1] = 2**31 - 2
+    fwd, inv = O.stwo_twiddles(log_n)
+    for row in x:
+        d = dev(row)
+        V.lib().cuda_stwo_ntt_evaluate(ptr(d), ptr(dev(fwd)), 1 << log_n)
+        assert np.array_equal(host(d), O.stwo_evaluate(row, log_n))
+        V.lib().cuda_stwo_ntt_interpolate(ptr(d), ptr(dev(inv)), 1 << log_n)
+        assert np.array_equal(host(d), row)
+    dst = empty(2 << (log_n + 2))
+    V.check(V.lib().vs_lde_stwo(ptr(dev(x.reshape(-1))), 1 << log_n, ptr(dst), 4 << log_n, 2, log_n, 2, None), "vs_lde_stwo")
+    assert np.array_equal(host(dst).reshape(2, -1), O.stwo_lde_columns(x, log_n, 2, threads=8))

@@ -57,27 +57,34 @@ __device__ __forceinline__ uint32_t swz(uint32_t a) {
   return a ^ (h << 2);
 }
 
-// x * t mod p from tt = 2t (< 2^32): x * tt = hi * 2^32 + lo with lo even, so
-// x * t = hi * 2^31 + lo / 2 == hi + lo / 2 (mod p), and both halves are < 2^31.
-// Written as one 64-bit product, so both halves come from a single wide multiply
-// (as two 32-bit multiplies the LDE of 34 x 2^24 took 18.2 ms; 16.8 ms like this).
+// Inside a pass a word is any representative in [-p, p), as a signed integer; tile stores
+// reduce to [0, p).
+__device__ __forceinline__ uint32_t lift(uint32_t x) { return min(x, x + VS_P); }  // [-p, p) -> [0, p)
+__device__ __forceinline__ uint4 lift(uint4 v) { return make_uint4(lift(v.x), lift(v.y), lift(v.z), lift(v.w)); }
+// Twiddles are centred and doubled: tt = 2t', t' == t with |t'| < p/2.
+__device__ __forceinline__ uint32_t twice(uint32_t t) { return (t + (t >> 30)) << 1; }
+// x * t mod p in [-p, p) for x in [-p, p): x * tt = hi * 2^32 + lo with lo a signed 32-bit
+// number and even, so x * t = hi * 2^31 + lo / 2 == hi + lo / 2 (mod p), |hi| and |lo / 2| at
+// most 2^30. The wide multiply's addend 2^31 rounds hi for the signed lo and leaves
+// lo + 2^31 below; its -2^62 takes the 2^30 of (lo + 2^31) / 2 off again. No reduction follows.
 __device__ __forceinline__ uint32_t mul_tt(uint32_t x, uint32_t tt) {
-  const uint64_t p = (uint64_t)x * tt;  // one wide multiply gives both halves
-  return canon((uint32_t)(p >> 32) + ((uint32_t)p >> 1));
+  const uint64_t p = (uint64_t)((int64_t)(int32_t)x * (int32_t)tt) + 0xC000000080000000ull;
+  return (uint32_t)(p >> 32) + ((uint32_t)p >> 1);
 }
 
-// Butterflies take doubled twiddles (tt = 2t).
+// A sum stays below p by taking p off in the same three-operand addition, a difference of
+// words in [0, p) is in range by itself: two reductions a butterfly, of its two inputs (or
+// of the product), where keeping every word in [0, p) takes three. The passes are bound by
+// integer issue (ALU and wide-multiply pipes both about 65 % busy): the lower pass executes
+// 9.76 instructions a butterfly instead of 10.25, and the LDE of 34 x 2^20 takes 747 us
+// instead of 768, of 34 x 2^22 3.09 ms instead of 3.18, of 34 x 2^24 14.43 instead of 14.60.
+// (The product's addend as a register pair of a fused wide multiply-add costs two more
+// instructions, 908 us; rounding with a compare instead, 833-942 us.)
 template <bool FWD>
 __device__ __forceinline__ void bfly(uint32_t& v0, uint32_t& v1, uint32_t tt) {
-  if (FWD) {
-    uint32_t m = mul_tt(v1, tt);
-    v1 = sub(v0, m);
-    v0 = add(v0, m);
-  } else {
-    uint32_t s = v0;
-    v0 = add(s, v1);
-    v1 = mul_tt(sub(s, v1), tt);
-  }
+  const uint32_t a = lift(v0), b = lift(FWD ? mul_tt(v1, tt) : v1);
+  v0 = a + b - VS_P;
+  v1 = FWD ? a - b : mul_tt(a - b, tt);
 }
 
 __device__ __forceinline__ uint32_t smem_addr(const void* p) {
@@ -153,7 +160,7 @@ __device__ __forceinline__ void tile_store(const uint32_t* sm, uint32_t* __restr
 #pragma unroll
   for (int i = 0; i < S::SIZE / 4 / S::NT; i++) {
     const uint32_t e = 4 * (threadIdx.x + i * S::NT);
-    *reinterpret_cast<uint4*>(dst + gidx<M, C>(g, e)) = *reinterpret_cast<const uint4*>(sm + swz<C>(e));
+    *reinterpret_cast<uint4*>(dst + gidx<M, C>(g, e)) = lift(*reinterpret_cast<const uint4*>(sm + swz<C>(e)));
   }
 }
 
@@ -228,10 +235,10 @@ __device__ __forceinline__ void rbfly(uint32_t (&v)[32], const TileGeo& g, const
         for (int gg = 0; gg < (K >> 1); gg += 4) {  // hb is a multiple of 4 here
           const uint32_t pr = 2 * ((hb >> 2) + (gg >> 2));
           const uint32_t x = __ldg(tw.flat + pr), y = __ldg(tw.flat + pr + 1);
-          t[gg] = y << 1;
-          t[gg + 1] = neg(y) << 1;
-          t[gg + 2] = neg(x) << 1;
-          t[gg + 3] = x << 1;
+          t[gg] = twice(y);
+          t[gg + 1] = 0u - twice(y);
+          t[gg + 2] = 0u - twice(x);
+          t[gg + 3] = twice(x);
         }
       } else {
         // A thread's twiddles of one layer are consecutive and start at a
@@ -244,18 +251,18 @@ __device__ __forceinline__ void rbfly(uint32_t (&v)[32], const TileGeo& g, const
 #pragma unroll
           for (int v = 0; v < cnt / 4; v++) {
             const uint4 w = __ldg(reinterpret_cast<const uint4*>(tp) + v);
-            t[o + 4 * v] = w.x << 1;
-            t[o + 4 * v + 1] = w.y << 1;
-            t[o + 4 * v + 2] = w.z << 1;
-            t[o + 4 * v + 3] = w.w << 1;
+            t[o + 4 * v] = twice(w.x);
+            t[o + 4 * v + 1] = twice(w.y);
+            t[o + 4 * v + 2] = twice(w.z);
+            t[o + 4 * v + 3] = twice(w.w);
           }
         } else if (cnt == 2) {
           const uint2 w = __ldg(reinterpret_cast<const uint2*>(tp));
-          t[o] = w.x << 1;
-          t[o + 1] = w.y << 1;
+          t[o] = twice(w.x);
+          t[o + 1] = twice(w.y);
         } else {
 #pragma unroll
-          for (int gg = 0; gg < cnt; gg++) t[o + gg] = __ldg(tp + gg) << 1;
+          for (int gg = 0; gg < cnt; gg++) t[o + gg] = twice(__ldg(tp + gg));
         }
       }
     }
@@ -283,7 +290,7 @@ __device__ __forceinline__ void round_sm(uint32_t* sm, const TileGeo& g, const N
   rbfly<FWD, M, C, r>(v, g, tw);
   if (scale) {
 #pragma unroll
-    for (int k = 0; k < 32; k++) v[k] = mul(v[k], scale);
+    for (int k = 0; k < 32; k++) v[k] = mul_tt(v[k], twice(scale));
   }
   rstore<M, C, r>(v, sm);
 }
@@ -373,7 +380,7 @@ __global__ void __launch_bounds__(1 << (M + C - 5), 2) ntt_lde_top_kernel(NttPas
     rload<M, C, TOP>(v, sm);
     rbfly<false, M, C, TOP>(v, gi, inv.tw);
 #pragma unroll
-    for (int k = 0; k < 32; k++) v[k] = mul(v[k], inv.scale);
+    for (int k = 0; k < 32; k++) v[k] = mul_tt(v[k], twice(inv.scale));
     rstore<M, C, TOP>(v, cf);
   }
   __syncthreads();
@@ -458,22 +465,22 @@ __device__ __forceinline__ void small_tw(uint32_t (&t)[8], const TileGeo& g, con
       const uint32_t* tp = tw.layer[g.a + p - C] + hb;
       if (p == 0 && tw.stwo && g.a == 0) {  // [y, -y, -x, x] of one pair of line layer 0
         const uint2 w = __ldg(reinterpret_cast<const uint2*>(tw.flat) + (hb >> 2));
-        t[o] = w.y << 1;
-        t[o + 1] = neg(w.y) << 1;
-        t[o + 2] = neg(w.x) << 1;
-        t[o + 3] = w.x << 1;
+        t[o] = twice(w.y);
+        t[o + 1] = 0u - twice(w.y);
+        t[o + 2] = 0u - twice(w.x);
+        t[o + 3] = twice(w.x);
       } else if (cnt == 4) {
         const uint4 w = __ldg(reinterpret_cast<const uint4*>(tp));
-        t[o] = w.x << 1;
-        t[o + 1] = w.y << 1;
-        t[o + 2] = w.z << 1;
-        t[o + 3] = w.w << 1;
+        t[o] = twice(w.x);
+        t[o + 1] = twice(w.y);
+        t[o + 2] = twice(w.z);
+        t[o + 3] = twice(w.w);
       } else if (cnt == 2) {
         const uint2 w = __ldg(reinterpret_cast<const uint2*>(tp));
-        t[o] = w.x << 1;
-        t[o + 1] = w.y << 1;
+        t[o] = twice(w.x);
+        t[o + 1] = twice(w.y);
       } else {
-        t[o] = __ldg(tp) << 1;
+        t[o] = twice(__ldg(tp));
       }
     }
   }
@@ -580,10 +587,12 @@ __global__ void __launch_bounds__(Small<M, C>::NT) ntt_pass_small_kernel(NttPass
     small_inv<M, C, 0, false>(v, t, small_sm, g, p.tw, g, p.tw);
     if (p.scale) {
 #pragma unroll
-      for (int k = 0; k < 8; k++) v[k] = mul(v[k], p.scale);
+      for (int k = 0; k < 8; k++) v[k] = mul_tt(v[k], twice(p.scale));
     }
   }
   uint32_t* dst = col_dst(p, col);
+#pragma unroll
+  for (int k = 0; k < 8; k++) v[k] = lift(v[k]);
   small_move<M, C, LAST, true>(v, [&](uint32_t e) { return dst + gidx<M, C>(g, e); });
 }
 // The LDE's top pass in this form: one CTA per (tile, column, blowup block), each doing the
@@ -608,12 +617,14 @@ __global__ void __launch_bounds__(Small<M, C>::NT) ntt_lde_top_small_kernel(NttP
   small_inv<M, C, 0, true>(v, t, small_sm, gi, inv.tw, gf, fwd.tw);
   cluster_arrive();  // this thread's words of the tile are read
 #pragma unroll
-  for (int k = 0; k < 8; k++) v[k] = mul(v[k], inv.scale);
+  for (int k = 0; k < 8; k++) v[k] = lift(mul_tt(v[k], twice(inv.scale)));
   if (inv.dst && q == 0) {  // the caller keeps the coefficients too
     uint32_t* cd = col_dst(inv, col);
     small_move<M, C, TOP, true>(v, [&](uint32_t e) { return cd + gidx<M, C>(gi, e); });
   }
   small_fwd<M, C, TOP>(v, t, small_sm, gf, fwd.tw);
+#pragma unroll
+  for (int k = 0; k < 8; k++) v[k] = lift(v[k]);
   cluster_wait();
   uint32_t* dst = col_dst(fwd, col);
   small_move<M, C, 0, true>(v, [&](uint32_t e) { return dst + gidx<M, C>(gf, e); });
@@ -689,7 +700,7 @@ __device__ __forceinline__ void tile_store4(const uint32_t* sm, uint32_t* __rest
 #pragma unroll
   for (int i = 0; i < S::SIZE / 4 / S::NT; i++) {
     const uint32_t e = 4 * (threadIdx.x + i * S::NT);
-    *reinterpret_cast<uint4*>(dst + gidx<M, C>(g, e)) = *reinterpret_cast<const uint4*>(sm + swz<0>(e));
+    *reinterpret_cast<uint4*>(dst + gidx<M, C>(g, e)) = lift(*reinterpret_cast<const uint4*>(sm + swz<0>(e)));
   }
 }
 // Tile store of a cluster of K CTAs over adjacent tiles lo0 .. lo0+K-1: each tile
@@ -713,7 +724,7 @@ __device__ __forceinline__ void tile_store4_cluster(const uint32_t* sm, uint32_t
     const uint32_t p = threadIdx.x + i * S::NT;  // chunk of this CTA's share
     const uint32_t j = p % SEG, r = rank * (R / K) + p / SEG;
     const uint32_t e = (r << C) | ((j % CH) << 2);  // tile word of chunk j % CH of row r
-    const uint4 v = ld_cluster16(cluster_peer(sm0 + 4 * swz<0>(e), j / CH));
+    const uint4 v = lift(ld_cluster16(cluster_peer(sm0 + 4 * swz<0>(e), j / CH)));
     *reinterpret_cast<uint4*>(dst + (base | (r << g.a) | (j << 2))) = v;
   }
 }
@@ -769,16 +780,16 @@ __device__ __forceinline__ void tw4_fetch(uint32_t (&t)[8], const TileGeo& g, co
       const int cnt = K >> (q + 1), o = s * (K - 1) + K - (K >> q);
       if (cnt == 4) {
         const uint4 w = __ldg(reinterpret_cast<const uint4*>(tp));
-        t[o] = w.x << 1;
-        t[o + 1] = w.y << 1;
-        t[o + 2] = w.z << 1;
-        t[o + 3] = w.w << 1;
+        t[o] = twice(w.x);
+        t[o + 1] = twice(w.y);
+        t[o + 2] = twice(w.z);
+        t[o + 3] = twice(w.w);
       } else if (cnt == 2) {
         const uint2 w = __ldg(reinterpret_cast<const uint2*>(tp));
-        t[o] = w.x << 1;
-        t[o + 1] = w.y << 1;
+        t[o] = twice(w.x);
+        t[o + 1] = twice(w.y);
       } else {
-        t[o] = __ldg(tp) << 1;
+        t[o] = twice(__ldg(tp));
       }
     }
   }
@@ -825,10 +836,10 @@ __device__ __forceinline__ void inv_rounds4(uint32_t* sm, uint32_t* cf, const Ti
     if (scale) {
 #pragma unroll
       for (int k = 0; k < 8; k++) {
-        v[k].x = mul(v[k].x, scale);
-        v[k].y = mul(v[k].y, scale);
-        v[k].z = mul(v[k].z, scale);
-        v[k].w = mul(v[k].w, scale);
+        v[k].x = mul_tt(v[k].x, twice(scale));
+        v[k].y = mul_tt(v[k].y, twice(scale));
+        v[k].z = mul_tt(v[k].z, twice(scale));
+        v[k].w = mul_tt(v[k].w, twice(scale));
       }
     }
     rstore4<M, C, r, S0>(v, cf);
@@ -967,10 +978,10 @@ __device__ __forceinline__ void round4(uint32_t* sm, const TileGeo& g, const Ntt
   if (scale) {
 #pragma unroll
     for (int k = 0; k < 8; k++) {
-      v[k].x = mul(v[k].x, scale);
-      v[k].y = mul(v[k].y, scale);
-      v[k].z = mul(v[k].z, scale);
-      v[k].w = mul(v[k].w, scale);
+      v[k].x = mul_tt(v[k].x, twice(scale));
+      v[k].y = mul_tt(v[k].y, twice(scale));
+      v[k].z = mul_tt(v[k].z, twice(scale));
+      v[k].w = mul_tt(v[k].w, twice(scale));
     }
   }
   rstore4<M, C, r, S0>(v, sm);
@@ -1198,9 +1209,9 @@ __global__ void ntt_layer_kernel(uint32_t* __restrict__ d, NttTw tw, uint32_t j,
   uint32_t h = tid >> j, l = tid & ((1u << j) - 1);
   uint32_t i0 = (h << (j + 1)) + l, i1 = i0 + (1u << j);
   uint32_t v0 = d[i0], v1 = d[i1];
-  bfly<FWD>(v0, v1, twiddle(tw, j, h) << 1);
-  d[i0] = v0;
-  d[i1] = v1;
+  bfly<FWD>(v0, v1, twice(twiddle(tw, j, h)));
+  d[i0] = lift(v0);
+  d[i1] = lift(v1);
 }
 __global__ void scale_kernel(uint32_t* __restrict__ d, uint32_t s, uint32_t n) {
   uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
