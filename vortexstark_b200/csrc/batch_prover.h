@@ -27,7 +27,7 @@ class BatchProver {
   // runs at the next of those sizes, the extra proofs being discarded).
   int init(uint32_t log_n, uint32_t capacity);
   // Starts proofs of (ab[2i], ab[2i+1]) for i < count <= capacity on stream `on`
-  // (one batch in flight per instance); finish() waits and serialises each proof.
+  // (one batch in flight per instance); finish() waits and copies each proof.
   int launch(const uint32_t* ab, uint32_t count, cudaStream_t on);
   int finish(std::vector<std::vector<uint8_t>>& out);
   // One proof on `st`, as a batch of one without a workspace kept (stream-ordered

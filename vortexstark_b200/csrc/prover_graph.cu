@@ -7,7 +7,7 @@
 // (values + authentication paths, one CTA per query recomputing its 1024-leaf
 // tile) writes straight into a proof arena that is copied to pinned host memory
 // once. A proof is therefore a single graph launch; the host only writes (a, b)
-// and serialises the arena (KRAK v1, src/bin/stark_cli.rs:907-976).
+// and copies the proof out of the arena (KRAK v1, src/bin/stark_cli.rs:907-976).
 //
 // Slots: each GraphProver owns its buffers, stream and graph, so several slots
 // prove concurrently (the batched and served paths).

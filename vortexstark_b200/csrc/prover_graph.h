@@ -39,7 +39,7 @@ class GraphProver {
   // numbers are served first when several streams have work queued).
   int init(uint32_t log_n, int priority = 0);
   // Starts a proof (one in flight per instance) on `on` (default: the prover's own
-  // stream); finish() waits for it and serialises KRAK v1.
+  // stream); finish() waits for it and copies the proof (KRAK v1).
   int launch(uint32_t a, uint32_t b, cudaStream_t on = nullptr);
   int finish(uint32_t a, uint32_t b, std::vector<uint8_t>& out);
   bool busy() const;
