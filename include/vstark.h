@@ -290,8 +290,8 @@ int vs_merkle_root_rowpacked(const uint32_t* d_cols, uint64_t stride, uint32_t n
  * allocation failure or sync). No counterpart in the reference. Accepts at most
  * 2^26 leaves (VS_ERR_INVALID beyond). The first call on a device, and the first
  * after the device's context was recreated, looks up the array's device address;
- * make it before any stream capture. All calls share the array: calls whose work
- * overlaps on the GPU race. */
+ * make it before any stream capture. All calls above 1024 leaves share the array:
+ * such calls whose work overlaps on the GPU race. */
 int vs_merkle_root_rowpacked_noalloc(const uint32_t* d_cols, uint64_t stride, uint32_t n_cols, uint32_t log_leaves,
                                      uint32_t* d_root, vs_stream_t stream);
 /* Merkle root with the reference's <=16-column leaf (blake2s.cu leaf semantics). */

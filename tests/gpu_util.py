@@ -81,3 +81,64 @@ def qm_mul(x, y):
 
 def qm_add(x, y):
     return [(int(a) + int(b)) % P for a, b in zip(x, y)]
+
+
+# --- driver calls of the tests on captured graphs and small memory pools
+def _cu(name, *args):
+    rc = getattr(C.CDLL("libcuda.so.1"), name)(*args)
+    assert rc == 0, f"{name}: {rc}"
+
+
+class _KernelNode(C.Structure):
+    _fields_ = [("func", C.c_void_p), ("grid", C.c_uint * 3), ("block", C.c_uint * 3), ("smem", C.c_uint),
+                ("params", C.c_void_p), ("extra", C.c_void_p), ("kern", C.c_void_p), ("ctx", C.c_void_p)]
+
+
+def captured(call):
+    """What call(stream handle) enqueues, as a capture sees it: the sorted (grid, block) of its
+    kernels, and its number of memory nodes (stream-ordered allocations and frees)."""
+    s = torch.cuda.Stream()
+    st, graph, n = C.c_void_p(s.cuda_stream), C.c_void_p(), C.c_size_t()
+    _cu("cuStreamBeginCapture_v2", st, 1)  # errors of this thread only
+    try:
+        call(s.cuda_stream)
+    finally:
+        _cu("cuStreamEndCapture", st, C.byref(graph))
+    _cu("cuGraphGetNodes", graph, None, C.byref(n))
+    nodes = (C.c_void_p * n.value)()
+    _cu("cuGraphGetNodes", graph, nodes, C.byref(n))
+    kernels, memory = [], 0
+    for node in nodes:
+        kind, k = C.c_int(), _KernelNode()
+        _cu("cuGraphNodeGetType", C.c_void_p(node), C.byref(kind))
+        memory += kind.value in (10, 11)  # CU_GRAPH_NODE_TYPE_MEM_ALLOC, _MEM_FREE
+        if kind.value == 0:
+            _cu("cuGraphKernelNodeGetParams_v2", C.c_void_p(node), C.byref(k))
+            kernels.append((tuple(k.grid), tuple(k.block)))
+    _cu("cuGraphDestroy", graph)
+    return sorted(kernels), memory
+
+
+class _PoolProps(C.Structure):
+    _fields_ = [("alloc_type", C.c_int), ("handle_types", C.c_int), ("location_type", C.c_int), ("device", C.c_int),
+                ("win32", C.c_void_p), ("max_size", C.c_size_t), ("usage", C.c_ushort), ("reserved", C.c_ubyte * 54)]
+
+
+class small_pool:
+    """Stream-ordered allocations come from a pool of at most max_bytes; larger ones fail."""
+
+    def __init__(self, max_bytes):
+        self.props = _PoolProps(alloc_type=1, location_type=1, device=torch.cuda.current_device(), max_size=max_bytes)
+
+    def __enter__(self):
+        torch.cuda.synchronize()
+        self.dev, self.old, self.pool = self.props.device, C.c_void_p(), C.c_void_p()
+        _cu("cuDeviceGetMemPool", C.byref(self.old), self.dev)
+        _cu("cuMemPoolCreate", C.byref(self.pool), C.byref(self.props))
+        _cu("cuDeviceSetMemPool", self.dev, self.pool)
+        return self
+
+    def __exit__(self, *exc):
+        torch.cuda.synchronize()
+        _cu("cuDeviceSetMemPool", self.dev, self.old)
+        _cu("cuMemPoolDestroy", self.pool)

@@ -16,13 +16,14 @@
 
 namespace vs {
 
-// Largest tree this entry point accepts, and the scratch that tree needs: one
-// 8-word subtree root per 1024 leaves plus the next reduction level.
+// Largest tree this entry point accepts, and the scratch that it needs at split 0: 2^16
+// roots of 1024 leaves, then 2^7 of 512 of those. Smaller trees take as wide a first
+// level as fits.
 constexpr uint32_t NOALLOC_MAX_LOG_LEAVES = 26;
 constexpr uint64_t NOALLOC_SCRATCH_WORDS = ((1ull << (NOALLOC_MAX_LOG_LEAVES - 10)) + 128) * 8;  // 2.1 MB
 
 // Every GPU that loads the library holds this array until the process exits.
-// All calls on a device share it and it keeps the last call's contents; calls
+// All calls above 1024 leaves share it on a device and it keeps the last call's contents; calls
 // whose work overlaps on the GPU would race on it.
 static __device__ __align__(256) uint32_t g_noalloc_scratch[NOALLOC_SCRATCH_WORDS];
 
@@ -103,13 +104,17 @@ extern "C" int vs_merkle_root_rowpacked_noalloc(const uint32_t* d_cols, uint64_t
                      "vs_merkle_root_rowpacked_noalloc: 2^%u leaves exceeds the fixed scratch limit of 2^%u leaves",
                      log_leaves, NOALLOC_MAX_LOG_LEAVES);
   const uint64_t n = 1ull << log_leaves;
-  uint32_t* scratch = nullptr;  // trees of at most 1024 leaves need no scratch
+  const LeafRowPacked leaf{d_cols, stride, n_cols};
+  // One CTA up to 1024 leaves: the array stays out of it, so such calls may overlap
+  // (at 2^10 leaves of 34 columns 34.9 us; two launches through the array 22.0).
+  if (log_leaves <= MK_MAX_TL) return merkle_tile_roots(leaf, n, log_leaves, d_root, (cudaStream_t)st);
+  uint32_t* scratch = nullptr;
   uint32_t split = merkle_root_split(log_leaves);  // as wide a first level as the array holds
   while (split && merkle_scratch_words(n, split) > NOALLOC_SCRATCH_WORDS) split--;
   if (merkle_scratch_words(n, split) > NOALLOC_SCRATCH_WORDS)
     return set_error(VS_ERR_INVALID, "vs_merkle_root_rowpacked_noalloc: scratch for 2^%u leaves exceeds the array",
                      log_leaves);
-  if (merkle_scratch_words(n, split) > 0) VS_TRY(noalloc_scratch(&scratch));
-  // With scratch supplied (or not needed) merkle_root performs no allocation.
-  return merkle_root(LeafRowPacked{d_cols, stride, n_cols}, n, d_root, (cudaStream_t)st, scratch, split);
+  VS_TRY(noalloc_scratch(&scratch));
+  // With scratch supplied merkle_root performs no allocation.
+  return merkle_root(leaf, n, d_root, (cudaStream_t)st, scratch, split);
 }
