@@ -1,11 +1,9 @@
 """What root-only trees take besides their input: nothing up to 1024 leaves where that matters
 (a capture, the variant without allocations), and no more than there is."""
-import ctypes as C
-
 import numpy as np
 import pytest
 
-from gpu_util import captured, dev, empty, host, ptr, small_pool, zeros
+from gpu_util import captured, dev, host, ptr, zeros
 
 pytestmark = pytest.mark.gpu
 
@@ -28,3 +26,25 @@ def test_noalloc_roots_up_to_1024_leaves_share_nothing(log_leaves):
     assert len(kernels) == 1 and memory == 0
     V.check(V.lib().vs_merkle_root_rowpacked_noalloc(ptr(d), 1 << log_leaves, 3, log_leaves, ptr(root), None))
     assert np.array_equal(host(root), O.merkle_root_rowpacked(cols))
+
+
+def _launches(call):
+    before = V.lib().vs_launch_count()
+    call()
+    return V.lib().vs_launch_count() - before
+
+
+def test_trees_that_one_launch_ends():
+    """2^9 leaves, and 2^10 hashes: a second launch costs more than it saves."""
+    L = V.lib()
+    cols, d = _cols(9)
+    root = zeros(8)
+    assert _launches(lambda: V.check(L.vs_merkle_root_rowpacked(ptr(d), 1 << 9, 3, 9, ptr(root), None))) == 1
+    assert np.array_equal(host(root), O.merkle_root_rowpacked(cols))
+    q = O.seeded_m31(0x55, 4 << 9).reshape(4, -1)
+    assert _launches(lambda: L.cuda_merkle_commit_small_soa4(*[ptr(dev(c)) for c in q], ptr(root), 1 << 9)) == 1
+    assert np.array_equal(host(root), O.merkle_root_soa4(q))
+    for log_n in (9, 10):
+        nodes = O.seeded_m31(0x66 + log_n, 8 << log_n)
+        assert _launches(lambda: L.cuda_merkle_reduce_to_root(ptr(dev(nodes)), ptr(root), 1 << log_n)) == 1
+        assert np.array_equal(host(root), O.merkle_root_hashes(nodes.reshape(-1, 8)))

@@ -5,6 +5,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <type_traits>
 
 #include "merkle_impl.cuh"
 #include "vs_common.cuh"
@@ -54,13 +55,15 @@ inline uint32_t merkle_root_split(uint32_t L) {
 // Tile of a reduction level over 2^L leaves, or over 2^L hashes of the level before:
 // 2^TL of them, reduced to 2^stop. Measured on whole roots (us, one 1024-leaf tile a CTA
 // and one root a tile, then this rule; 34 / 16 columns): 2^12 leaves 43 -> 23 / 31 -> 23,
-// 2^16 46 -> 33 / 36 -> 29, 2^18 74 -> 68 / 51 -> 47, 2^19 132 -> 109 / 84 -> 70.
+// 2^16 46 -> 33 / 36 -> 29, 2^18 74 -> 68 / 51 -> 47, 2^19 132 -> 109 / 84 -> 70. One CTA
+// ends trees of up to 2^9 leaves (14.4 us with one column, 22.5 with 34; tiles of 2^7 and a
+// second launch 18.5 and 22.5) and of 2^10 hashes (14.9; 16.4).
 // Split 0, for callers with little scratch, leaves one root a tile from 2^18 on.
 struct MerkleTile {
   uint32_t TL, stop;
 };
 inline MerkleTile merkle_tile(uint32_t L, bool hashes, uint32_t split) {
-  if (L <= (hashes ? 10u : 8u)) return {L, 0};
+  if (L <= (hashes ? 10u : 9u)) return {L, 0};
   if (L <= 14) return {7, 0};
   if (L <= 17) return {L - 7, 0};
   if (L < MK_WIDE) return split ? MerkleTile{L - 10, 7} : MerkleTile{MK_MAX_TL, 0};
@@ -85,11 +88,11 @@ int merkle_forest(const MerkleForest& f, uint32_t TL, cudaStream_t st) {
 
 // Words of scratch merkle_root needs for n_leaves leaves with split `split` (0 when
 // one CTA does): the sum of the hash levels it writes, in the order it writes them
-// (merkle_root follows the same sequence).
-inline uint64_t merkle_scratch_words(uint64_t n_leaves, uint32_t split = 0) {
+// (merkle_root follows the same sequence). hashes: the leaves are hashes already.
+inline uint64_t merkle_scratch_words(uint64_t n_leaves, uint32_t split = 0, bool hashes = false) {
   uint64_t words = 0;
   uint32_t L = ilog2(n_leaves);
-  for (bool hashes = false;; hashes = true) {
+  for (;; hashes = true) {
     const MerkleTile t = merkle_tile(L, hashes, split);
     if (t.TL == L && !t.stop) return words;
     L -= t.TL - t.stop;
@@ -142,14 +145,15 @@ int merkle_root(const Leaf& leaf, uint64_t n_leaves, uint32_t* d_root, cudaStrea
   if (!is_pow2(n_leaves)) return set_error(VS_ERR_INVALID, "merkle: leaf count %llu is not a power of two",
                                            (unsigned long long)n_leaves);
   if (split > MK_MAX_SPLIT) return set_error(VS_ERR_INVALID, "merkle: split %u above %u", split, MK_MAX_SPLIT);
-  const uint64_t words = merkle_scratch_words(n_leaves, split);
+  constexpr bool hashes = std::is_same_v<Leaf, LeafHashes>;
+  const uint64_t words = merkle_scratch_words(n_leaves, split, hashes);
   uint32_t *level = scratch, *buf = nullptr;
   if (words && !scratch) {
     VS_CUDA(cudaMallocAsync((void**)&buf, words * 4, st));
     level = buf;
   }
   uint32_t L = ilog2(n_leaves);
-  MerkleTile t = merkle_tile(L, false, split);
+  MerkleTile t = merkle_tile(L, hashes, split);
   bool last = t.TL == L && !t.stop;
   int rc = merkle_tile_roots(leaf, n_leaves, t.TL, last ? d_root : level, st, t.stop);
   while (rc == VS_OK && !last) {
