@@ -264,9 +264,15 @@ int vs_autotune_lde(uint32_t log_n, uint32_t n_cols, uint32_t blowup_bits, uint3
  * the first reduction level stops at 2^split roots per 1024-leaf tile (0..8), so a
  * CTA skips the narrow top levels of its tile, and the next level reduces them; 0,
  * the default, leaves the choice to the library, and trees below 2^20 leaves take
- * smaller tiles of their own. Roots are identical for every split. Process wide; applies to vs_commit_columns,
- * vs_merkle_root_rowpacked / _capped / _soa4, vs_fri_fold_commit, the Cairo FRI and
- * the engine's commitment jobs (their scratch is sized for split 8). */
+ * smaller tiles of their own. Roots are identical for every split. Process wide; applies
+ * to vs_commit_columns, vs_merkle_root_rowpacked / _capped / _soa4, vs_fri_fold_commit and
+ * the engine's commitment jobs (their scratch is sized for split 8), and caps the subtree
+ * roots per tile of trees that keep their tile roots (the graph prover, the Cairo
+ * commitments).
+ * Scratch of a root-only tree, stream-ordered for the call: 32 bytes for each of those
+ * roots and for each of the levels above that is written (by default 4 MB at 2^20 leaves,
+ * 306 MB at 2^26, less above). Where it cannot be allocated the tree leaves one root a
+ * 1024-leaf tile instead, slower and with 32 bytes a tile. */
 int vs_merkle_split_set(uint32_t split);
 uint32_t vs_merkle_split_get(void);
 /* Times the row-packed root of n_cols seeded columns x 2^log_leaves rows (11..28) at

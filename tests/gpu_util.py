@@ -125,10 +125,12 @@ class _PoolProps(C.Structure):
 
 
 class small_pool:
-    """Stream-ordered allocations come from a pool of at most max_bytes; larger ones fail."""
+    """Stream-ordered allocations come from a pool of at most max_bytes (in steps of 32 MB);
+    what does not fit fails."""
 
     def __init__(self, max_bytes):
         self.props = _PoolProps(alloc_type=1, location_type=1, device=torch.cuda.current_device(), max_size=max_bytes)
+        self.held = None
 
     def __enter__(self):
         torch.cuda.synchronize()
@@ -138,7 +140,15 @@ class small_pool:
         _cu("cuDeviceSetMemPool", self.dev, self.pool)
         return self
 
+    def hold(self, n_bytes):
+        """Takes n_bytes of the pool until the end."""
+        self.held = C.c_void_p()
+        _cu("cuMemAllocAsync", C.byref(self.held), C.c_size_t(n_bytes), None)
+
     def __exit__(self, *exc):
         torch.cuda.synchronize()
+        if self.held:
+            _cu("cuMemFreeAsync", self.held, None)
+            torch.cuda.synchronize()
         _cu("cuDeviceSetMemPool", self.dev, self.old)
         _cu("cuMemPoolDestroy", self.pool)

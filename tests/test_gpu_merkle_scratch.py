@@ -3,7 +3,7 @@
 import numpy as np
 import pytest
 
-from gpu_util import captured, dev, host, ptr, zeros
+from gpu_util import captured, dev, host, ptr, small_pool, zeros
 
 pytestmark = pytest.mark.gpu
 
@@ -48,3 +48,18 @@ def test_trees_that_one_launch_ends():
         nodes = O.seeded_m31(0x66 + log_n, 8 << log_n)
         assert _launches(lambda: L.cuda_merkle_reduce_to_root(ptr(dev(nodes)), ptr(root), 1 << log_n)) == 1
         assert np.array_equal(host(root), O.merkle_root_hashes(nodes.reshape(-1, 8)))
+
+
+@pytest.mark.parametrize("log_leaves,held", [(24, 0), (10, 32 << 20)])
+def test_roots_where_scratch_cannot_be_allocated(log_leaves, held):
+    """The default split's 80 MB at 2^24 leaves, and any scratch at 2^10: the tree then leaves one
+    root a tile, which takes 0.5 MB and none."""
+    n = 1 << log_leaves
+    d, root, less = zeros(n), zeros(8), zeros(8)
+    V.check(V.lib().vs_fill_uniform_m31(ptr(d), n, 7, 0, None))
+    V.check(V.lib().vs_merkle_root_rowpacked(ptr(d), n, 1, log_leaves, ptr(root), None))
+    with small_pool(32 << 20) as pool:
+        if held:
+            pool.hold(held)
+        V.check(V.lib().vs_merkle_root_rowpacked(ptr(d), n, 1, log_leaves, ptr(less), None))
+    assert np.array_equal(host(less), host(root))

@@ -58,11 +58,14 @@ inline uint32_t merkle_root_split(uint32_t L) {
 // 2^16 46 -> 33 / 36 -> 29, 2^18 74 -> 68 / 51 -> 47, 2^19 132 -> 109 / 84 -> 70. One CTA
 // ends trees of up to 2^9 leaves (14.4 us with one column, 22.5 with 34; tiles of 2^7 and a
 // second launch 18.5 and 22.5) and of 2^10 hashes (14.9; 16.4).
-// Split 0, for callers with little scratch, leaves one root a tile from 2^18 on.
+// Split 0, for callers with little scratch, leaves one root a tile from 2^18 on;
+// MK_LEAST does at every size, which takes the least scratch (none up to 2^10 leaves).
+constexpr uint32_t MK_LEAST = MK_MAX_SPLIT + 1;
 struct MerkleTile {
   uint32_t TL, stop;
 };
 inline MerkleTile merkle_tile(uint32_t L, bool hashes, uint32_t split) {
+  if (split == MK_LEAST) return {std::min<uint32_t>(L, MK_MAX_TL), 0};
   if (L <= (hashes ? 10u : 9u)) return {L, 0};
   if (L <= 14) return {7, 0};
   if (L <= 17) return {L - 7, 0};
@@ -136,8 +139,8 @@ inline uint64_t merkle_scratch_words_any(uint64_t n_leaves) {
 
 // Root of a power-of-two tree whose leaves come from `leaf`. Intermediate tile
 // roots go to `scratch` (merkle_scratch_words(n_leaves, split) words; when null it
-// is allocated stream-ordered for the call). Each reduction level is written after
-// the previous one, never in place. Levels of 2^MK_WIDE and more stop at 2^split roots
+// is allocated stream-ordered for the call; where that fails the tree is built with
+// MK_LEAST instead). Each reduction level is written after the previous one, never in place. Levels of 2^MK_WIDE and more stop at 2^split roots
 // per 1024-leaf tile (split <= MK_MAX_SPLIT); the root is the same for every split.
 template <class Leaf>
 int merkle_root(const Leaf& leaf, uint64_t n_leaves, uint32_t* d_root, cudaStream_t st, uint32_t* scratch = nullptr,
@@ -146,10 +149,18 @@ int merkle_root(const Leaf& leaf, uint64_t n_leaves, uint32_t* d_root, cudaStrea
                                            (unsigned long long)n_leaves);
   if (split > MK_MAX_SPLIT) return set_error(VS_ERR_INVALID, "merkle: split %u above %u", split, MK_MAX_SPLIT);
   constexpr bool hashes = std::is_same_v<Leaf, LeafHashes>;
-  const uint64_t words = merkle_scratch_words(n_leaves, split, hashes);
+  uint64_t words = merkle_scratch_words(n_leaves, split, hashes);
   uint32_t *level = scratch, *buf = nullptr;
   if (words && !scratch) {
-    VS_CUDA(cudaMallocAsync((void**)&buf, words * 4, st));
+    cudaError_t e = cudaMallocAsync((void**)&buf, words * 4, st);
+    if (e == cudaErrorMemoryAllocation) {
+      cudaGetLastError();  // the refused allocation's error
+      buf = nullptr;
+      split = MK_LEAST;
+      words = merkle_scratch_words(n_leaves, split, hashes);
+      e = words ? cudaMallocAsync((void**)&buf, words * 4, st) : cudaSuccess;
+    }
+    VS_TRY(check_cuda(e, "merkle scratch"));
     level = buf;
   }
   uint32_t L = ilog2(n_leaves);
