@@ -63,3 +63,10 @@ def test_roots_where_scratch_cannot_be_allocated(log_leaves, held):
             pool.hold(held)
         V.check(V.lib().vs_merkle_root_rowpacked(ptr(d), n, 1, log_leaves, ptr(less), None))
     assert np.array_equal(host(less), host(root))
+
+
+def test_captured_roots_up_to_1024_leaves_have_no_memory_nodes():
+    cols, d = _cols(10)
+    root = zeros(8)
+    kernels, memory = captured(lambda st: V.check(V.lib().vs_merkle_root_rowpacked(ptr(d), 1 << 10, 3, 10, ptr(root), st)))
+    assert len(kernels) == 1 and memory == 0

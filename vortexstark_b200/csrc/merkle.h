@@ -149,6 +149,11 @@ int merkle_root(const Leaf& leaf, uint64_t n_leaves, uint32_t* d_root, cudaStrea
                                            (unsigned long long)n_leaves);
   if (split > MK_MAX_SPLIT) return set_error(VS_ERR_INVALID, "merkle: split %u above %u", split, MK_MAX_SPLIT);
   constexpr bool hashes = std::is_same_v<Leaf, LeafHashes>;
+  // A capture of a tree of one tile stays free of memory nodes, so that its graph may be
+  // instantiated and launched more than once.
+  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+  if (!scratch && n_leaves <= (1ull << MK_MAX_TL) && cudaStreamIsCapturing(st, &capture) != cudaSuccess) cudaGetLastError();
+  if (capture != cudaStreamCaptureStatusNone) split = MK_LEAST;
   uint64_t words = merkle_scratch_words(n_leaves, split, hashes);
   uint32_t *level = scratch, *buf = nullptr;
   if (words && !scratch) {
