@@ -837,7 +837,7 @@ def main():
     ach = alg["merkle"] / (phase["merkle"] / 1e3) / 1e9
     roof = {"bound": "hbm", "kernel": "merkle_subtree_kernel<LeafRowPacked>", "achieved": ach, "peak": hbm,
             "peak_source": hbm_src, "unit": "GB/s", "frac": ach / hbm,
-            "traffic": alg["merkle"] * 1.0004 + (N >> 10 << api.merkle_split()) * 32,
+            "traffic": alg["merkle"] * 1.0004 + (N >> 10 << (api.merkle_split() or 7)) * 32,
             "algorithmic_bytes": alg["merkle"],
             # The binding resource is integer issue: instructions per launch (1179
             # per Blake2s compression on average, the ncu count of this kernel at

@@ -276,10 +276,12 @@ int vs_autotune_lde(uint32_t log_n, uint32_t n_cols, uint32_t blowup_bits, uint3
 int vs_merkle_split_set(uint32_t split);
 uint32_t vs_merkle_split_get(void);
 /* Times the row-packed root of n_cols seeded columns x 2^log_leaves rows (11..28) at
- * every split (one warm-up and `reps` timed runs each, CUDA events on `stream`),
+ * every split 1..8 (one warm-up and `reps` timed runs each, CUDA events on `stream`),
  * checks that all splits give one root, keeps the fastest split and writes it to
- * *best; ms[s] (s < cap) receives split s's time per root. Allocates its scratch on
- * `stream`. */
+ * *best; ms[s] (s < cap) receives split s's time per root, ms[0] that of the library's
+ * own choice, and 0 is kept where that is the fastest. Below 2^20 leaves every split
+ * runs the same tiles: the split stays as it was set, and every ms[s] is that one time.
+ * Allocates its scratch on `stream`. */
 int vs_autotune_merkle(uint32_t log_leaves, uint32_t n_cols, uint32_t reps, uint32_t* best, float* ms, uint32_t cap,
                        vs_stream_t stream);
 

@@ -129,6 +129,23 @@ def test_autotune_merkle_keeps_a_split(L, default_split):
     assert all(t > 0 for t in res["ms"]) and res["ms"][res["best"]] == min(res["ms"])
 
 
+@pytest.mark.parametrize("log_leaves", [11, 17, 18, 19])
+def test_autotune_merkle_leaves_the_split_where_it_is_not_used(L, default_split, log_leaves):
+    api.set_merkle_split(6)
+    res = api.autotune_merkle(log_leaves, n_cols=3, reps=1)
+    assert res["best"] == 6 == api.merkle_split()
+    assert len(set(res["ms"])) == 1
+
+
+def test_autotune_merkle_reports_the_split_that_runs(L, default_split):
+    """Split 0 is the library's choice (7 here), timed as such: what is kept is what was measured."""
+    for _ in range(3):
+        api.set_merkle_split(0)
+        res = api.autotune_merkle(21, n_cols=2, reps=3)
+        assert res["ms"][0] == res["ms"][7]
+        assert res["ms"][res["best"]] == min(res["ms"]) and api.merkle_split() == res["best"] != 7
+
+
 @pytest.mark.parametrize("split", [1, 5, 8])
 def test_prover_trees_with_split_match_oracle(L, default_split, split):
     """Proof trees of 2^20 leaves (log_n 18) go through 2^min(split, 5) subtree

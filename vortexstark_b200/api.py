@@ -151,7 +151,8 @@ def autotune_lde(log_n: int, n_cols: int = 34, blowup: int = 2, reps: int = 3, s
 
 
 def merkle_split() -> int:
-    """First-level split of root-only Merkle trees (2^split roots per 1024-leaf tile)."""
+    """First-level split of root-only Merkle trees of 2^20 leaves and more (2^split roots per
+    1024-leaf tile); 0: the library's choice."""
     return int(lib().vs_merkle_split_get())
 
 
@@ -160,7 +161,8 @@ def set_merkle_split(split: int) -> None:
 
 
 def autotune_merkle(log_leaves: int, n_cols: int = 34, reps: int = 3, stream=None) -> dict:
-    """Times the row-packed root at every split, keeps the fastest; {"best": s, "ms": [...]}."""
+    """Times the row-packed root at every split and keeps the fastest; {"best": s, "ms": [...]}.
+    ms[0] is the library's choice. Below 2^20 leaves all splits are the same and none is set."""
     best = C.c_uint32()
     ms = (C.c_float * 9)()
     check(lib().vs_autotune_merkle(log_leaves, n_cols, reps, C.byref(best), ms, 9, _stream(stream)),

@@ -172,8 +172,10 @@ int vs_merkle_split_set(uint32_t split) {
 uint32_t vs_merkle_split_get(void) { return merkle_split(); }
 
 // Times the row-packed root of n_cols seeded columns of 2^log_leaves rows at every
-// split (one warm-up and `reps` timed runs each, CUDA events on the stream), checks
-// that every split gives the same root, and keeps the fastest split.
+// split from 1 on (one warm-up and `reps` timed runs each, CUDA events on the stream),
+// checks that every split gives the same root, and keeps the fastest split; 0 when that
+// is the library's own choice, whose time it reports for split 0. Trees below 2^MK_WIDE
+// leaves have the same tiles at every split: one is timed and the split is left as it is.
 int vs_autotune_merkle(uint32_t log_leaves, uint32_t n_cols, uint32_t reps, uint32_t* best, float* ms_out, uint32_t cap,
                        vs_stream_t stream) {
   clear_error();
@@ -191,9 +193,10 @@ int vs_autotune_merkle(uint32_t log_leaves, uint32_t n_cols, uint32_t reps, uint
   if (rc == VS_OK) rc = vs_fill_uniform_m31(cols, n * n_cols, 0x56530008ull, 0, stream);
   if (rc == VS_OK) rc = check_cuda(cudaEventCreate(&e0), "vs_autotune_merkle event");
   if (rc == VS_OK) rc = check_cuda(cudaEventCreate(&e1), "vs_autotune_merkle event");
-  uint32_t best_split = merkle_split();
-  float best_ms = 0.f;
-  for (uint32_t sp = 0; sp <= MK_MAX_SPLIT && rc == VS_OK; sp++) {
+  const bool wide = log_leaves >= MK_WIDE;
+  const uint32_t own = merkle_default_split(log_leaves), most = wide ? MK_MAX_SPLIT : 1;
+  float split_ms[MK_MAX_SPLIT + 1] = {};
+  for (uint32_t sp = 1; sp <= most && rc == VS_OK; sp++) {
     const LeafRowPacked leaf{cols, n, n_cols};
     rc = merkle_root(leaf, n, roots + 8 * sp, st, scratch, sp);
     if (rc == VS_OK) rc = check_cuda(cudaEventRecord(e0, st), "vs_autotune_merkle event");
@@ -202,25 +205,27 @@ int vs_autotune_merkle(uint32_t log_leaves, uint32_t n_cols, uint32_t reps, uint
     if (rc == VS_OK) rc = check_cuda(cudaEventSynchronize(e1), "vs_autotune_merkle sync");
     float ms = 0.f;
     if (rc == VS_OK) rc = check_cuda(cudaEventElapsedTime(&ms, e0, e1), "vs_autotune_merkle time");
-    ms /= (float)reps;
-    if (ms_out && sp < cap) ms_out[sp] = ms;
-    if (rc == VS_OK && (sp == 0 || ms < best_ms)) {
-      best_ms = ms;
-      best_split = sp;
-    }
+    split_ms[sp] = ms / (float)reps;
+  }
+  split_ms[0] = split_ms[wide ? own : 1];
+  uint32_t best_split = wide ? 0 : merkle_split();
+  for (uint32_t sp = 0; sp <= MK_MAX_SPLIT && rc == VS_OK; sp++) {
+    if (!wide) split_ms[sp] = split_ms[0];
+    else if (split_ms[sp] < split_ms[best_split]) best_split = sp;
+    if (ms_out && sp < cap) ms_out[sp] = split_ms[sp];
   }
   uint32_t h[8 * (MK_MAX_SPLIT + 1)];
   if (rc == VS_OK) rc = check_cuda(cudaMemcpyAsync(h, roots, sizeof(h), cudaMemcpyDeviceToHost, st), "vs_autotune_merkle copy");
   if (rc == VS_OK) rc = check_cuda(cudaStreamSynchronize(st), "vs_autotune_merkle sync");
-  for (uint32_t sp = 1; sp <= MK_MAX_SPLIT && rc == VS_OK; sp++)
-    if (memcmp(h, h + 8 * sp, 32) != 0) rc = set_error(VS_ERR_CUDA, "vs_autotune_merkle: split %u gave another root", sp);
+  for (uint32_t sp = 2; sp <= most && rc == VS_OK; sp++)
+    if (memcmp(h + 8, h + 8 * sp, 32) != 0) rc = set_error(VS_ERR_CUDA, "vs_autotune_merkle: split %u gave another root", sp);
   if (e0) cudaEventDestroy(e0);
   if (e1) cudaEventDestroy(e1);
   if (cols) cudaFreeAsync(cols, st);
   if (scratch) cudaFreeAsync(scratch, st);
   if (roots) cudaFreeAsync(roots, st);
   if (rc != VS_OK) return rc;
-  g_merkle_split.store(best_split);
+  if (wide) g_merkle_split.store(best_split);
   *best = best_split;
   return check_cuda(cudaStreamSynchronize(st), "vs_autotune_merkle");
 }

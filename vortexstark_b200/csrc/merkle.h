@@ -48,9 +48,10 @@ constexpr uint32_t MK_WIDE = 20;
 // Split of a wide tree of 2^L leaves when none is set: 7, the fastest (row-packed root
 // of 34 x 2^26: 11.90 / 11.64 / 11.30 / 11.42 ms at 5 / 6 / 7 / 8), less where its
 // roots would take more than 256 MB of scratch.
+inline uint32_t merkle_default_split(uint32_t L) { return L <= 26 ? 7u : 33u - L; }
 inline uint32_t merkle_root_split(uint32_t L) {
   const uint32_t s = merkle_split();
-  return s ? s : (L <= 26 ? 7u : 33u - L);
+  return s ? s : merkle_default_split(L);
 }
 // Tile of a reduction level over 2^L leaves, or over 2^L hashes of the level before:
 // 2^TL of them, reduced to 2^stop. Measured on whole roots (us, one 1024-leaf tile a CTA
