@@ -331,3 +331,23 @@ def test_group_commit_tile_roots_with_split(L, split):
     finally:
         api.set_merkle_split(0)
     check(got, O.commit_group_cairo(cols, log_n, blind))
+
+
+def test_group_commit_where_scratch_cannot_be_allocated(L):
+    """2^24 evaluation rows take 64 MB for the subtree roots of their tiles by default; without
+    room for them beside the 16 MB canonic copy the tile roots come without a split."""
+    from gpu_util import small_pool
+    log_n = 22
+    n, N = 1 << log_n, 4 << log_n
+    cols, ev, root, tiles = empty(n), empty(N), empty(8), empty(N // 1024 * 8)
+    V.check(L.vs_fill_uniform_m31(ptr(cols), n, 11, 0, None))
+
+    def commit():
+        rc = L.vs_commit_group_cairo(ptr(cols), n, 1, log_n, None, None, ptr(ev), None, ptr(root), ptr(tiles), None)
+        assert rc == 0, L.vs_last_error()
+        return host(root), host(tiles)
+
+    exp = commit()
+    with small_pool(64 << 20):
+        got = commit()
+    assert all(np.array_equal(a, b) for a, b in zip(got, exp))

@@ -590,12 +590,22 @@ int eval_at_points(const uint32_t* const* h_cols, uint32_t n_cols, uint32_t L, c
   return VS_OK;
 }
 
-// 1024-leaf tile roots of a commitment (merkle_tile_roots_split); stream-ordered scratch.
+// 1024-leaf tile roots of a commitment (merkle_tile_roots_split); stream-ordered scratch of
+// at most 256 MB, and none (one root a tile) where it cannot be allocated.
 template <class Leaf>
 int tile_roots_split(const Leaf& leaf, uint64_t N, uint32_t* tiles, cudaStream_t st) {
-  const uint32_t sp = merkle_tile_split(N, MK_MAX_SPLIT);
+  uint32_t sp = std::min(merkle_tile_split(N, MK_MAX_SPLIT), 33 - std::min(ilog2(N), 33u));
   uint32_t* sub = nullptr;
-  if (sp) VS_CUDA(cudaMallocAsync((void**)&sub, merkle_tile_scratch_bytes(N, sp), st));
+  if (sp) {
+    const cudaError_t e = cudaMallocAsync((void**)&sub, merkle_tile_scratch_bytes(N, sp), st);
+    if (e == cudaErrorMemoryAllocation) {
+      cudaGetLastError();  // the refused allocation's error
+      sub = nullptr;
+      sp = 0;
+    } else {
+      VS_TRY(check_cuda(e, "subtree roots"));
+    }
+  }
   const int rc = merkle_tile_roots_split(leaf, N, MK_MAX_TL, sp, tiles, sub, st);
   if (sub) cudaFreeAsync(sub, st);
   return rc;
@@ -993,20 +1003,20 @@ extern "C" int vs_cairo_oods_fri(void* channel, vs_cairo_oods_fri_io* io, vs_str
     VS_TRY(get_fold_twiddles(l == 0 ? (int)FOLD_CANONIC_CIRCLE : (int)COSET_HALF_ODDS, log_eval - l, &tws[l], st));
   uint32_t* otiles = io->oods_tile_roots;
   if (!otiles) VS_TRY(s.alloc(&otiles, n_tiles * 8));
-  auto tree = [&](uint32_t m, TreeLevels* t) {  // levels kept only to be taken up by the next launch
-    *t = TreeLevels{nullptr, 1, m >= MK_WIDE ? 5u : channel_leaf_tile(m, m), m};
+  auto tree = [&](uint32_t m, uint32_t from, TreeLevels* t) {  // levels kept only to be taken up by the next launch
+    *t = TreeLevels{nullptr, 1, from, m};
     return s.alloc(&t->base, TreeLevels::bytes(1, t->s, m) / 4);
   };
   const LeafSoa4 oleaf{oq[0], oq[1], oq[2], oq[3]};
+  auto lowest = [](uint32_t m) { return m >= MK_WIDE ? 5u : channel_leaf_tile(m, m); };
   TreeLevels lv{};
-  VS_TRY(tree(log_eval, &lv));
+  VS_TRY(tree(log_eval, N <= 1024 ? lowest(log_eval) : MK_MAX_TL, &lv));
   if (N <= 1024) {
     VS_TRY(commit_with_channel(oleaf, lv, 1, after(0), st));
     VS_CUDA(cudaMemcpyAsync(otiles, d_tr->roots, 32, cudaMemcpyDeviceToDevice, st));
   } else {
     VS_TRY(tile_roots_split(oleaf, N, otiles, st));
     const uint32_t TL = std::min<uint32_t>(MK_MAX_TL, log_eval - MK_MAX_TL);
-    lv.s = MK_MAX_TL;
     VS_TRY(channel_tiles(LeafHashes{otiles}, lv, MK_MAX_TL, TL, 1, after(0), st));
     VS_TRY(channel_levels(lv, MK_MAX_TL + TL, 1, after(0), st));
   }
@@ -1024,7 +1034,7 @@ extern "C" int vs_cairo_oods_fri(void* channel, vs_cairo_oods_fri_io* io, vs_str
     tail.tw[l] = tws[l];
     tail.tree[l] = TreeLevels{nullptr, 1, 32, m};  // no level is kept (32 is above every level)
     if (m > TAIL_LOG) {
-      VS_TRY(tree(m, &lv));
+      VS_TRY(tree(m, lowest(m), &lv));
       VS_TRY(commit_with_channel(LeafFoldAt{src, dst, tws[l], d_tr->alphas + 4 * l}, lv, 1, after(1 + l), st));
       for (int k = 0; k < 4; k++) src.c[k] = dst.c[k];
     } else if (l < tail.first) {
