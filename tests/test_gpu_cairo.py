@@ -351,3 +351,21 @@ def test_group_commit_where_scratch_cannot_be_allocated(L):
     with small_pool(64 << 20):
         got = commit()
     assert all(np.array_equal(a, b) for a, b in zip(got, exp))
+
+
+def test_cairo_tail_columns_at_one_stride_off_a_boundary(L):
+    """Interaction columns and quotient limbs at one stride, from a 16-byte boundary (one launch,
+    no copies) and from one word after it (copies), give the same tail."""
+    from vortexstark_b200 import api
+    log_n, ni = 12, 9
+    n, N = 1 << log_n, 4 << log_n
+    trace, evals = api.fill_uniform_m31(empty(2 * n), seed=1), api.fill_uniform_m31(empty(2 * N), seed=2)
+    cols = api.fill_uniform_m31(empty((ni + 4) * N), seed=5)
+
+    def tail(shift):
+        buf = empty((ni + 4) * N + 4)
+        c = buf[shift:shift + (ni + 4) * N].copy_(cols).reshape(ni + 4, N)
+        return api.cairo_oods_fri(api.Channel(), log_n, list(trace.reshape(2, n)), list(evals.reshape(2, N)),
+                                  list(c[:ni]), list(c[ni:]))
+
+    assert tail(1) == tail(0) == tail(2)

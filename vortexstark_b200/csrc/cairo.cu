@@ -739,10 +739,13 @@ std::vector<h::Q> line_coeffs_from_evals(std::vector<h::Q> e) {
   brev_all(e);
   return e;
 }
-// Whether n columns of at least N words start at one positive stride (16-byte aligned
-// columns then take no copies on their way into a transform).
+// Whether n columns of at least N words start on 16-byte boundaries at one positive stride:
+// they then move in one launch, and into a transform without copies (others would be copied
+// on its way in and again on its way out).
 bool even_stride(const uint32_t* const* cols, uint32_t n, uint64_t N, uint64_t* stride) {
   *stride = N;
+  for (uint32_t j = 0; j < n; j++)
+    if (reinterpret_cast<uintptr_t>(cols[j]) & 15) return false;
   if (n < 2) return true;
   if (cols[1] < cols[0]) return false;
   *stride = cols[1] - cols[0];
