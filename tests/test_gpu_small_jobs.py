@@ -89,3 +89,18 @@ def test_edge_values_through_every_pass_form(log_n):
     dst = empty(2 << (log_n + 2))
     V.check(V.lib().vs_lde_stwo(ptr(dev(x.reshape(-1))), 1 << log_n, ptr(dst), 4 << log_n, 2, log_n, 2, None), "vs_lde_stwo")
     assert np.array_equal(host(dst).reshape(2, -1), O.stwo_lde_columns(x, log_n, 2, threads=8))
+
+
+@pytest.mark.parametrize("log_n", list(range(5, 14)))
+def test_word_round_lde(log_n):
+    """Blowups above 8 run in word rounds, on plain words up to 12 layers and signed words at 13;
+    words at the ends of [0, p), both conventions."""
+    n, N = 1 << log_n, 16 << log_n
+    x = EDGE[np.random.default_rng(log_n).integers(0, len(EDGE), (2, n))]
+    dst = empty(2 * N)
+    V.check(V.lib().vs_lde_stwo(ptr(dev(x.reshape(-1))), n, ptr(dst), N, 2, log_n, 4, None), "vs_lde_stwo")
+    assert np.array_equal(host(dst).reshape(2, N), O.stwo_lde_columns(x, log_n, 4, threads=8))
+    V.check(V.lib().vs_lde_native(ptr(dev(x.reshape(-1))), n, ptr(dst), N, 2, log_n, 4, None), "vs_lde_native")
+    for got, row in zip(host(dst).reshape(2, N), x):
+        coeffs = np.concatenate([O.native_interpolate(row, log_n), np.zeros(N - n, np.uint32)])
+        assert np.array_equal(got, O.native_evaluate(coeffs, log_n + 4))

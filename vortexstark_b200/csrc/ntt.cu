@@ -86,6 +86,34 @@ __device__ __forceinline__ void bfly(uint32_t& v0, uint32_t& v1, uint32_t tt) {
   v0 = a + b - VS_P;
   v1 = FWD ? a - b : mul_tt(a - b, tt);
 }
+// The same on words in [0, p), with plainly doubled twiddles (tt = 2t < 2^32; x * tt = hi *
+// 2^32 + lo, x * t == hi + lo / 2): three reductions a butterfly, but one operation less a
+// twiddle and none at a tile's store. Words (`SW` below: signed words) are kept like this
+// where a twiddle serves few butterflies of a thread and few tiles share an SM: the LDEs of
+// at most 12 layers in word rounds (signed words, then plain, us: 1 x 2^12 x16 51.4 -> 47.2,
+// native 53.4 -> 45.2, 8192 x 2^8 x16 native 269 -> 236; at 13 layers 73.8 -> 75.9).
+__device__ __forceinline__ uint32_t mul_tt_plain(uint32_t x, uint32_t tt) {
+  const uint64_t p = (uint64_t)x * tt;
+  return canon((uint32_t)(p >> 32) + ((uint32_t)p >> 1));
+}
+template <bool SW, bool FWD>
+__device__ __forceinline__ void word_bfly(uint32_t& v0, uint32_t& v1, uint32_t tt) {
+  if (SW) {
+    bfly<FWD>(v0, v1, tt);
+  } else if (FWD) {
+    const uint32_t m = mul_tt_plain(v1, tt);
+    v1 = sub(v0, m);
+    v0 = add(v0, m);
+  } else {
+    const uint32_t s = v0;
+    v0 = add(s, v1);
+    v1 = mul_tt_plain(sub(s, v1), tt);
+  }
+}
+template <bool SW>
+__device__ __forceinline__ uint32_t word_twice(uint32_t t) { return SW ? twice(t) : t << 1; }
+template <bool SW>
+__device__ __forceinline__ uint32_t word_mul(uint32_t x, uint32_t t) { return SW ? mul_tt(x, twice(t)) : mul(x, t); }
 
 __device__ __forceinline__ uint32_t smem_addr(const void* p) {
   return static_cast<uint32_t>(__cvta_generic_to_shared(p));
@@ -154,13 +182,14 @@ __device__ __forceinline__ void tile_load_async(uint32_t* sm, const uint32_t* __
     cp_async16(base + 4 * swz<C>(e), src + (gidx<M, C>(g, e) & mask));
   }
 }
-template <int M, int C>
+template <int M, int C, bool SW = true>
 __device__ __forceinline__ void tile_store(const uint32_t* sm, uint32_t* __restrict__ dst, const TileGeo& g) {
   using S = Tile<M, C>;
 #pragma unroll
   for (int i = 0; i < S::SIZE / 4 / S::NT; i++) {
     const uint32_t e = 4 * (threadIdx.x + i * S::NT);
-    *reinterpret_cast<uint4*>(dst + gidx<M, C>(g, e)) = lift(*reinterpret_cast<const uint4*>(sm + swz<C>(e)));
+    const uint4 v = *reinterpret_cast<const uint4*>(sm + swz<C>(e));
+    *reinterpret_cast<uint4*>(dst + gidx<M, C>(g, e)) = SW ? lift(v) : v;
   }
 }
 
@@ -215,7 +244,7 @@ __device__ __forceinline__ void rstore(const uint32_t (&v)[32], uint32_t* sm) {
 // fetched into registers first (doubled, for mul_tt) so their loads overlap
 // instead of stalling each butterfly. Layer at tile bit p = P0 + q is global layer j = a + p - C; its
 // group index is h = hi * 2^(T-1-p) + (address >> (p+1)).
-template <bool FWD, int M, int C, int r>
+template <bool FWD, int M, int C, int r, bool SW = true>
 __device__ __forceinline__ void rbfly(uint32_t (&v)[32], const TileGeo& g, const NttTw& tw) {
   using S = Tile<M, C>;
   constexpr int P0 = S::P0(r), R = S::R(r), K = 1 << R, SUB = 1 << (5 - R), T = S::T;
@@ -235,10 +264,10 @@ __device__ __forceinline__ void rbfly(uint32_t (&v)[32], const TileGeo& g, const
         for (int gg = 0; gg < (K >> 1); gg += 4) {  // hb is a multiple of 4 here
           const uint32_t pr = 2 * ((hb >> 2) + (gg >> 2));
           const uint32_t x = __ldg(tw.flat + pr), y = __ldg(tw.flat + pr + 1);
-          t[gg] = twice(y);
-          t[gg + 1] = 0u - twice(y);
-          t[gg + 2] = 0u - twice(x);
-          t[gg + 3] = twice(x);
+          t[gg] = word_twice<SW>(y);
+          t[gg + 1] = SW ? 0u - twice(y) : neg(y) << 1;
+          t[gg + 2] = SW ? 0u - twice(x) : neg(x) << 1;
+          t[gg + 3] = word_twice<SW>(x);
         }
       } else {
         // A thread's twiddles of one layer are consecutive and start at a
@@ -251,18 +280,18 @@ __device__ __forceinline__ void rbfly(uint32_t (&v)[32], const TileGeo& g, const
 #pragma unroll
           for (int v = 0; v < cnt / 4; v++) {
             const uint4 w = __ldg(reinterpret_cast<const uint4*>(tp) + v);
-            t[o + 4 * v] = twice(w.x);
-            t[o + 4 * v + 1] = twice(w.y);
-            t[o + 4 * v + 2] = twice(w.z);
-            t[o + 4 * v + 3] = twice(w.w);
+            t[o + 4 * v] = word_twice<SW>(w.x);
+            t[o + 4 * v + 1] = word_twice<SW>(w.y);
+            t[o + 4 * v + 2] = word_twice<SW>(w.z);
+            t[o + 4 * v + 3] = word_twice<SW>(w.w);
           }
         } else if (cnt == 2) {
           const uint2 w = __ldg(reinterpret_cast<const uint2*>(tp));
-          t[o] = twice(w.x);
-          t[o + 1] = twice(w.y);
+          t[o] = word_twice<SW>(w.x);
+          t[o + 1] = word_twice<SW>(w.y);
         } else {
 #pragma unroll
-          for (int gg = 0; gg < cnt; gg++) t[o + gg] = twice(__ldg(tp + gg));
+          for (int gg = 0; gg < cnt; gg++) t[o + gg] = word_twice<SW>(__ldg(tp + gg));
         }
       }
     }
@@ -275,7 +304,7 @@ __device__ __forceinline__ void rbfly(uint32_t (&v)[32], const TileGeo& g, const
 #pragma unroll
         for (int l = 0; l < (1 << q); l++) {
           const int k0 = (gg << (q + 1)) | l;
-          bfly<FWD>(v[s * K + k0], v[s * K + k0 + (1 << q)], tv);
+          word_bfly<SW, FWD>(v[s * K + k0], v[s * K + k0 + (1 << q)], tv);
         }
       }
     }
@@ -283,14 +312,14 @@ __device__ __forceinline__ void rbfly(uint32_t (&v)[32], const TileGeo& g, const
 }
 
 // One full round through shared memory (caller provides the barrier after).
-template <bool FWD, int M, int C, int r>
+template <bool FWD, int M, int C, int r, bool SW = true>
 __device__ __forceinline__ void round_sm(uint32_t* sm, const TileGeo& g, const NttTw& tw, uint32_t scale) {
   uint32_t v[32];
   rload<M, C, r>(v, sm);
-  rbfly<FWD, M, C, r>(v, g, tw);
+  rbfly<FWD, M, C, r, SW>(v, g, tw);
   if (scale) {
 #pragma unroll
-    for (int k = 0; k < 32; k++) v[k] = mul_tt(v[k], twice(scale));
+    for (int k = 0; k < 32; k++) v[k] = word_mul<SW>(v[k], scale);
   }
   rstore<M, C, r>(v, sm);
 }
@@ -345,15 +374,15 @@ __global__ void __launch_bounds__(1 << (M + C - 5), (FWD && C == 0) ? 3 : 2) ntt
   }
 }
 
-template <bool FWD, int M, int C>
+template <bool FWD, int M, int C, bool SW>
 __device__ __forceinline__ void rounds_below_top(uint32_t* sm, const TileGeo& g, const NttTw& tw) {
   // forward: rounds NR-2 .. 0 ; inverse: rounds 0 .. NR-2 (the top round is handled by the caller)
   using S = Tile<M, C>;
 #pragma unroll
   for (int rr = 0; rr + 1 < S::NR; rr++) {
     const int r = FWD ? S::NR - 2 - rr : rr;
-    if (r == 0) round_sm<FWD, M, C, 0>(sm, g, tw, 0);
-    else round_sm<FWD, M, C, (S::NR > 2 ? 1 : 0)>(sm, g, tw, 0);
+    if (r == 0) round_sm<FWD, M, C, 0, SW>(sm, g, tw, 0);
+    else round_sm<FWD, M, C, (S::NR > 2 ? 1 : 0), SW>(sm, g, tw, 0);
     __syncthreads();
   }
 }
@@ -368,19 +397,20 @@ template <int M, int C>
 __global__ void __launch_bounds__(1 << (M + C - 5), 2) ntt_lde_top_kernel(NttPass inv, NttPass fwd, uint32_t B) {
   using S = Tile<M, C>;
   constexpr int TOP = S::NR - 1;
+  constexpr bool SW = C != 0 || M == 13;
   extern __shared__ uint32_t lde_sm[];
   uint32_t* sm = lde_sm;              // working tile
   uint32_t* cf = lde_sm + S::SIZE;    // coefficients
   const TileGeo gi = tile_geo<M, C>(inv.a, blockIdx.x);
   tile_load<M, C>(sm, col_src(inv, blockIdx.y), gi, inv.src_mask);
   __syncthreads();
-  rounds_below_top<false, M, C>(sm, gi, inv.tw);
+  rounds_below_top<false, M, C, SW>(sm, gi, inv.tw);
   {
     uint32_t v[32];
     rload<M, C, TOP>(v, sm);
-    rbfly<false, M, C, TOP>(v, gi, inv.tw);
+    rbfly<false, M, C, TOP, SW>(v, gi, inv.tw);
 #pragma unroll
-    for (int k = 0; k < 32; k++) v[k] = mul_tt(v[k], twice(inv.scale));
+    for (int k = 0; k < 32; k++) v[k] = word_mul<SW>(v[k], inv.scale);
     rstore<M, C, TOP>(v, cf);
   }
   __syncthreads();
@@ -391,11 +421,11 @@ __global__ void __launch_bounds__(1 << (M + C - 5), 2) ntt_lde_top_kernel(NttPas
     gf.gbase = (q << (gi.a + M)) | gi.gbase;
     uint32_t v[32];
     rload<M, C, TOP>(v, cf);
-    rbfly<true, M, C, TOP>(v, gf, fwd.tw);
+    rbfly<true, M, C, TOP, SW>(v, gf, fwd.tw);
     rstore<M, C, TOP>(v, sm);  // the previous block's tile_store finished before the loop-end barrier
     __syncthreads();
-    rounds_below_top<true, M, C>(sm, gf, fwd.tw);
-    tile_store<M, C>(sm, dst, gf);
+    rounds_below_top<true, M, C, SW>(sm, gf, fwd.tw);
+    tile_store<M, C, SW>(sm, dst, gf);
     __syncthreads();
   }
 }
