@@ -3,7 +3,7 @@ words in the small-job passes, against the oracle."""
 import numpy as np
 import pytest
 
-from gpu_util import dev, empty, host, ptr, ptr_array, rand_m31, u32_host
+from gpu_util import captured, dev, empty, host, ptr, ptr_array, rand_m31, u32_host
 
 pytestmark = pytest.mark.gpu
 
@@ -15,8 +15,10 @@ def cases():
     for log_n in range(5, 14):
         for blowup in (0, 1, 3):
             yield log_n, blowup, 3
-    yield 13, 3, 64   # 2^22 evaluation words: the most of at most 13 layers
-    yield 13, 3, 65   # above 2^22 evaluation words
+    for log_n, blowup, most in ((13, 3, 37), (13, 0, 148), (12, 2, 96), (10, 1, 592), (5, 2, 1184), (7, 3, 3072),
+                                (14, 0, 40)):
+        yield log_n, blowup, most      # on either side of the columns it takes
+        yield log_n, blowup, most + 1
     yield 8, 4, 2     # more blocks than it takes
     yield 14, 2, 16   # 2^20 evaluation words: the most of a larger transform
     yield 14, 2, 17
@@ -37,6 +39,23 @@ def test_small_lde(log_n, blowup, n_cols):
     coeffs = O.native_interpolate(cols[0], log_n)
     exp = O.native_evaluate(np.concatenate([coeffs, np.zeros(N - n, np.uint32)]), log_n + blowup)
     assert np.array_equal(host(dst)[:N], exp)
+
+
+def _lde_launches(n_cols, log_n, blowup):
+    src, dst = empty(n_cols << log_n), empty(n_cols << (log_n + blowup))
+    lde = lambda st: V.check(V.lib().vs_lde_stwo(ptr(src), 1 << log_n, ptr(dst), 1 << (log_n + blowup), n_cols, log_n,
+                                                 blowup, st))
+    lde(None)  # tables are made outside a capture
+    return captured(lde)[0]
+
+
+def test_many_columns_run_in_word_rounds():
+    """One CTA of 2^(log_n - 5) threads a column, where that fills the chip (128 columns x4 at 2^13
+    rows: 26 us, and 45 in the small-job passes); eight words a thread and a CTA a block otherwise."""
+    assert _lde_launches(128, 13, 2) == [((1, 128, 1), (256, 1, 1))]
+    assert _lde_launches(34, 13, 2) == [((34, 4, 1), (1024, 1, 1))]
+    assert _lde_launches(128, 12, 3) == [((1, 128, 1), (128, 1, 1))]
+    assert _lde_launches(34, 12, 3) == [((34, 8, 1), (512, 1, 1))]
 
 
 @pytest.mark.parametrize("log_n", list(range(5, 21)))

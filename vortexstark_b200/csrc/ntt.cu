@@ -1254,12 +1254,27 @@ static const uint32_t kMinC = 2;   // >= 16-byte contiguous runs per tile row
 // Jobs of few words (all columns together) run in the small-job passes unless a plan was
 // set for their size. Measured (us, 8192-word tiles then small-job passes):
 //  * transforms: 2^14 21.6 -> 17.1, 2^19 23.9 -> 20.5, but 2^20 23.9 -> 25.7;
-//  * LDEs of at most 13 layers, by evaluation words: 34 x 2^10 x4 (2^17) 16.8 -> 7.5,
-//    34 x 2^13 x8 (2^21) 43.5 -> 22.9;
+//  * LDEs of at most 13 layers: 34 x 2^10 x4 14.4 -> 5.8, 34 x 2^13 x8 43.0 -> 32.9;
 //  * LDEs above: 2 x 2^14 x4 24.9 -> 17.1, 4 x 2^16 x4 (2^20) 27.0 -> 22.9, 2 x 2^18 x2
 //    (2^20) 25.7 -> 23.0, but 7 x 2^17 x2 (1.75 x 2^20) 29.1 -> 29.2 and 34 x 2^14 x2
 //    (1.06 x 2^20) 23.0 -> 25.0: the repeated inverse layers then cost more than the
-//    idle SMs they fill.
+//    idle SMs they fill. LDEs without a blowup repeat none, but 48 x 2^14 (3 x 2^18) takes
+//    21.6 -> 22.8, 34 x 2^14 21.5 -> 18.5.
+// Most evaluation words of an LDE for that. Up to 13 layers the word rounds run a column's
+// blocks one after the other in one CTA, so many columns fill the chip and leave nothing to
+// gain: from ten layers on the line lies at one wave of 1024-thread CTAs up to x2 (148 x
+// 2^12 x2 14.4 -> 12.4 us, 160 x 2^12 x2 14.6 -> 16.5), 1.3 at x4 (96 x 2^12 x4 18.5 -> 16.5,
+// 112 columns 18.5 -> 20.6) and two at x8 (34 x 2^13 x8 43.0 -> 32.9, 48 columns 43.1 ->
+// 43.1). Smaller transforms leave lanes idle in the word rounds (512 x 2^9 x4 14.4 -> 9.3,
+// 768 x 2^9 x8 24.7 -> 20.6, 1024 columns 24.7 -> 26.7), but the 4-thread CTAs of 2^5 rows
+// stop at 32 an SM (1024 x 2^5 x4 10.3 either way, 4096 columns 24.7 -> 30.8).
+static uint64_t small_lde_words(uint32_t l, uint32_t B) {
+  constexpr uint64_t wave = 148ull << 13;
+  if (l > 13) return B ? 1ull << 20 : 5ull << 17;
+  if (l == 5 && B > 1) return wave >> 3;
+  if (l < 10 || (B == 0 && l < 13)) return B == 3 ? 3ull << 20 : 1ull << 22;
+  return B == 3 ? 2 * wave : B == 2 ? 3ull << 19 : wave;
+}
 static bool default_plan(uint32_t L) {
   const NttPlan p = ntt_plan(L);
   return p.lower == 0 && p.items == 0 && p.radix == 3;
@@ -1268,8 +1283,7 @@ static bool small_transform_job(uint32_t L, uint64_t words) {
   return L >= 5 && L <= kSmallMaxL && words <= (1ull << 19) && default_plan(L);
 }
 static bool small_lde_job(uint32_t l, uint32_t B, uint32_t n_cols) {
-  const uint64_t words = (uint64_t)n_cols << (l + B);
-  return l >= 5 && l <= kSmallMaxL && B <= 3 && words <= (l <= 13 ? 1ull << 22 : 1ull << 20) && default_plan(l);
+  return l >= 5 && l <= kSmallMaxL && B <= 3 && (uint64_t)n_cols << (l + B) <= small_lde_words(l, B) && default_plan(l);
 }
 // Lower (C = 0) and upper pass of a small transform of L layers; one pass up to 13.
 static std::vector<PassRange> small_passes(uint32_t L) {
