@@ -236,8 +236,9 @@ int vs_lde_native(const uint32_t* d_src, uint64_t src_stride, uint32_t* d_dst, u
 
 /* NTT launch-shape autotuner (no counterpart in the reference, which launches one
  * kernel per butterfly layer). A plan per transform size log_n (process wide, used
- * by every NTT and LDE of that size, native and stwo; an LDE uses the plan of its
- * trace size):
+ * by the NTTs and LDEs of that size, native and stwo; an LDE uses the plan of its
+ * trace size; jobs of few words in all, at most 2^19 in an NTT and about 2^20 evaluations
+ * in an LDE, run in passes of their own instead):
  *   lower      layers of the first (lower) pass; 14 <= log_n <= 24 accepts
  *              max(5, log_n - 11) .. 13, other sizes only their default
  *              (13, or log_n below 14);

@@ -1,6 +1,7 @@
 """GPU checks of the NTT launch-shape autotuner: every candidate plan gives the
 oracle's LDE and NTT bit for bit (plans regroup layers into launches, nothing
-else), and the tuner keeps one of the candidates and leaves results unchanged."""
+else), and the tuner keeps one of the candidates and leaves results unchanged. Jobs
+here have the columns that take them past the small-job passes, which no plan moves."""
 import numpy as np
 import pytest
 
@@ -9,7 +10,7 @@ import oracle_lib as O
 pytestmark = pytest.mark.gpu
 
 torch = pytest.importorskip("torch")
-from gpu_util import dev, empty, host, ptr, rand_m31  # noqa: E402
+from gpu_util import captured, dev, empty, host, ptr, ptr_array, rand_m31, u32_host  # noqa: E402
 import vortexstark_b200 as V  # noqa: E402
 from vortexstark_b200 import api  # noqa: E402
 
@@ -38,10 +39,10 @@ def _lde(L, cols, log_n, native=False):
     return host(dst).reshape(n_cols, N)
 
 
-@pytest.mark.parametrize("log_n", [14, 16, 18])
-def test_every_candidate_plan_matches_oracle(L, log_n):
+@pytest.mark.parametrize("log_n,n_cols", [(14, 17), (16, 5), (18, 3)])
+def test_every_candidate_plan_matches_oracle(L, log_n, n_cols):
     rng = np.random.default_rng(700 + log_n)
-    cols = rand_m31(rng, 3, 1 << log_n)
+    cols = rand_m31(rng, n_cols, 1 << log_n)
     exp = O.stwo_lde_columns(cols, log_n, 2, threads=4)
     cands = api.ntt_plan_candidates(log_n)
     assert len(cands) >= 6
@@ -51,25 +52,46 @@ def test_every_candidate_plan_matches_oracle(L, log_n):
         assert np.array_equal(_lde(L, cols, log_n), exp), plan
 
 
-@pytest.mark.parametrize("log_n", [15, 17])
-def test_plans_native_lde_and_transforms(L, log_n):
+@pytest.mark.parametrize("log_n,n_cols", [(15, 17), (17, 5)])
+def test_plans_native_lde_and_transforms(L, log_n, n_cols):
     rng = np.random.default_rng(800 + log_n)
-    x = rand_m31(rng, 1, 1 << log_n)
-    padded = np.zeros(1 << (log_n + 2), np.uint32)
-    padded[: 1 << log_n] = O.native_interpolate(x[0], log_n)
-    ref = O.native_evaluate(padded, log_n + 2)[None, :]
-    fwd_tw, inv_tw = O.stwo_twiddles(log_n)
-    exp_eval = O.stwo_evaluate(x[0], log_n)
+    x = rand_m31(rng, n_cols, 1 << log_n)
+    pad = np.zeros(3 << log_n, np.uint32)
+    ref = np.stack([O.native_evaluate(np.concatenate([O.native_interpolate(c, log_n), pad]), log_n + 2) for c in x])
+    exp_eval = [O.native_evaluate(c.copy(), log_n) for c in x]
+    tw = O.native_twiddles(log_n)
+
+    def batch(fn, cols, i=""):
+        fn(ptr(ptr_array(cols)), ptr(dev(tw[i + "line"])), ptr(dev(tw[i + "circle"])), u32_host(tw["offsets"]),
+           u32_host(tw["sizes"]), log_n - 1, 1 << log_n, n_cols)
+
     for plan in api.ntt_plan_candidates(log_n)[::5]:
         api.set_ntt_plan(log_n, *plan)
         assert np.array_equal(_lde(L, x, log_n, native=True), ref), plan
-        d = dev(x[0])
-        L.cuda_stwo_ntt_evaluate(ptr(d), ptr(dev(fwd_tw)), 1 << log_n)
-        assert np.array_equal(host(d), exp_eval), plan
-        L.cuda_stwo_ntt_interpolate(ptr(d), ptr(dev(inv_tw)), 1 << log_n)
-        assert np.array_equal(host(d), x[0]), plan
+        cols = [dev(c) for c in x]
+        batch(L.cuda_circle_ntt_evaluate_batch, cols)
+        assert all(np.array_equal(host(d), e) for d, e in zip(cols, exp_eval)), plan
+        batch(L.cuda_circle_ntt_interpolate_batch, cols, "i")
+        assert all(np.array_equal(host(d), c) for d, c in zip(cols, x)), plan
     api.set_ntt_plan(log_n)
     assert np.array_equal(_lde(L, x, log_n, native=True), ref)
+
+
+@pytest.mark.parametrize("log_n,n_cols,blowup", [(16, 1, 2), (14, 8, 1), (13, 34, 3), (8, 34, 2)])
+def test_tuning_a_size_leaves_its_small_jobs_alone(L, tmp_path, log_n, n_cols, blowup):
+    """A job of few words runs in the same launches after the size was tuned on 34 columns, and in
+    a process that loads the tuning."""
+    src, dst = empty(n_cols << log_n), empty(n_cols << (log_n + blowup))
+    lde = lambda st: V.check(L.vs_lde_stwo(ptr(src), 1 << log_n, ptr(dst), 1 << (log_n + blowup), n_cols, log_n,
+                                           blowup, st))
+    lde(None)
+    before = captured(lde)
+    api.autotune_lde(log_n, n_cols=34, reps=1)
+    assert captured(lde) == before
+    api.save_tuning(tmp_path / "t.json", [log_n])
+    api.set_ntt_plan(log_n)
+    api.load_tuning(tmp_path / "t.json")
+    assert captured(lde) == before
 
 
 def test_autotune_keeps_a_candidate_and_results(L):

@@ -1251,8 +1251,8 @@ __global__ void scale_kernel(uint32_t* __restrict__ d, uint32_t s, uint32_t n) {
 // ------------------------------------------------------------------ host side
 static const uint32_t kMaxT = 13;  // tile of 8192 words (32 KiB), 256 threads
 static const uint32_t kMinC = 2;   // >= 16-byte contiguous runs per tile row
-// Jobs of few words (all columns together) run in the small-job passes unless a plan was
-// set for their size. Measured (us, 8192-word tiles then small-job passes):
+// Jobs of few words (all columns together) run in the small-job passes, whatever the plan of
+// their size: that was tuned on, or set for, jobs that fill the chip. Measured (us, 8192-word tiles then small-job passes):
 //  * transforms: 2^14 21.6 -> 17.1, 2^19 23.9 -> 20.5, but 2^20 23.9 -> 25.7;
 //  * LDEs of at most 13 layers: 34 x 2^10 x4 14.4 -> 5.8, 34 x 2^13 x8 43.0 -> 32.9;
 //  * LDEs above: 2 x 2^14 x4 24.9 -> 17.1, 4 x 2^16 x4 (2^20) 27.0 -> 22.9, 2 x 2^18 x2
@@ -1280,10 +1280,15 @@ static bool default_plan(uint32_t L) {
   return p.lower == 0 && p.items == 0 && p.radix == 3;
 }
 static bool small_transform_job(uint32_t L, uint64_t words) {
-  return L >= 5 && L <= kSmallMaxL && words <= (1ull << 19) && default_plan(L);
+  return L >= 5 && L <= kSmallMaxL && words <= (1ull << 19);
 }
 static bool small_lde_job(uint32_t l, uint32_t B, uint32_t n_cols) {
-  return l >= 5 && l <= kSmallMaxL && B <= 3 && (uint64_t)n_cols << (l + B) <= small_lde_words(l, B) && default_plan(l);
+  uint64_t most = small_lde_words(l, B);
+  // The best plan of a size beats the small-job passes only near their line, at small
+  // blowups (us, best plan and small: 32 x 2^14 x2 18.5 / 22.6, 10 x 2^16 18.5 / 20.5; but
+  // 2^19 20.5 / 19.5, 4 x 2^16 x4 24.6 / 20.5, 16 x 2^14 x4 22.1 / 20.6).
+  if (l > 13 && B < 2 && !default_plan(l)) most = std::min<uint64_t>(most, 1ull << 19);
+  return l >= 5 && l <= kSmallMaxL && B <= 3 && (uint64_t)n_cols << (l + B) <= most;
 }
 // Lower (C = 0) and upper pass of a small transform of L layers; one pass up to 13.
 static std::vector<PassRange> small_passes(uint32_t L) {
@@ -1584,10 +1589,11 @@ static int ntt_transform_aligned(const NttColumns& io, uint32_t L, const NttTw& 
 }
 
 static int ntt_lde_aligned(const NttColumns& io, uint32_t l, uint32_t B, const NttTw& tw_inv, const NttTw& tw_fwd,
-                           cudaStream_t st, uint32_t* coeffs = nullptr, uint64_t coeffs_stride = 0);
+                           cudaStream_t st, const NttPlan& plan, bool small, uint32_t* coeffs = nullptr,
+                           uint64_t coeffs_stride = 0);
 
 int ntt_lde(const NttColumns& io, uint32_t l, uint32_t B, const NttTw& tw_inv, const NttTw& tw_fwd,
-            cudaStream_t st, uint32_t* coeffs, uint64_t coeffs_stride) {
+            cudaStream_t st, uint32_t* coeffs, uint64_t coeffs_stride, bool plan_only) {
   if (l < 5) return set_error(VS_ERR_INVALID, "LDE needs log_n >= 5 (got %u)", l);
   if (io.src_cols || io.dst_cols) return set_error(VS_ERR_INVALID, "LDE takes strided columns");
   StreamScratch tmp(st);
@@ -1597,11 +1603,12 @@ int ntt_lde(const NttColumns& io, uint32_t l, uint32_t B, const NttTw& tw_inv, c
   // The chunk-round top pass has the coefficients in hand and stores them as well;
   // otherwise they are one more interpolation.
   const NttColumns cio{io.src, coeffs, nullptr, nullptr, io.src_stride, coeffs_stride, io.n_cols};
-  const bool with = coeffs && (l > kMaxT || small_lde_job(l, B, io.n_cols)) && ntt_plan(l).radix != 5 &&
-                    strided_aligned(cio) && strided_aligned(io);
+  const NttPlan plan = ntt_plan(l);
+  const bool small = !plan_only && small_lde_job(l, B, io.n_cols);
+  const bool with = coeffs && (small || (l > kMaxT && plan.radix != 5)) && strided_aligned(cio) && strided_aligned(io);
   if (coeffs && !with) VS_TRY(ntt_transform(cio, l, ti, false, st));
   if (strided_aligned(io))
-    return ntt_lde_aligned(io, l, B, ti, tf, st, with ? coeffs : nullptr, coeffs_stride);
+    return ntt_lde_aligned(io, l, B, ti, tf, st, plan, small, with ? coeffs : nullptr, coeffs_stride);
   const uint64_t n = 1ull << l, N = n << B;
   uint32_t *S = nullptr, *D = nullptr;
   VS_TRY(tmp.alloc(&S, n * io.n_cols));
@@ -1609,16 +1616,14 @@ int ntt_lde(const NttColumns& io, uint32_t l, uint32_t B, const NttTw& tw_inv, c
   for (uint32_t c = 0; c < io.n_cols; c++)
     VS_CUDA(cudaMemcpyAsync(S + c * n, io.src + c * io.src_stride, n * 4, cudaMemcpyDeviceToDevice, st));
   NttColumns tio{S, D, nullptr, nullptr, n, N, io.n_cols};
-  VS_TRY(ntt_lde_aligned(tio, l, B, ti, tf, st));
+  VS_TRY(ntt_lde_aligned(tio, l, B, ti, tf, st, plan, small));
   for (uint32_t c = 0; c < io.n_cols; c++)
     VS_CUDA(cudaMemcpyAsync(io.dst + c * io.dst_stride, D + c * N, N * 4, cudaMemcpyDeviceToDevice, st));
   return VS_OK;
 }
 
 static int ntt_lde_aligned(const NttColumns& io, uint32_t l, uint32_t B, const NttTw& tw_inv, const NttTw& tw_fwd,
-                           cudaStream_t st, uint32_t* coeffs, uint64_t coeffs_stride) {
-  const NttPlan plan = ntt_plan(l);
-  const bool small = small_lde_job(l, B, io.n_cols);
+                           cudaStream_t st, const NttPlan& plan, bool small, uint32_t* coeffs, uint64_t coeffs_stride) {
   const auto passes = small ? small_passes(l) : plan_passes(l, plan.lower);
   const size_t np = passes.size();
   // 1. inverse passes below the top one: src -> dst[0, n)
@@ -1767,7 +1772,8 @@ int tw_for(int kind, uint32_t L, bool forward, NttTw* out, cudaStream_t st) {
 }
 
 int lde_cached(int kind, const uint32_t* src, uint64_t src_stride, uint32_t* dst, uint64_t dst_stride,
-               uint32_t n_cols, uint32_t l, uint32_t B, cudaStream_t st, uint32_t* coeffs, uint64_t coeffs_stride) {
+               uint32_t n_cols, uint32_t l, uint32_t B, cudaStream_t st, uint32_t* coeffs, uint64_t coeffs_stride,
+               bool plan_only) {
   if (!src || !dst || n_cols == 0) return set_error(VS_ERR_INVALID, "lde: null argument");
   if (l < 2 || l + B > 30) return set_error(VS_ERR_INVALID, "lde: log_n %u + blowup %u out of range", l, B);
   NttTw ti, tf;
@@ -1788,7 +1794,7 @@ int lde_cached(int kind, const uint32_t* src, uint64_t src_stride, uint32_t* dst
     return VS_OK;
   }
   NttColumns io{src, dst, nullptr, nullptr, src_stride, dst_stride, n_cols};
-  return ntt_lde(io, l, B, ti, tf, st, coeffs, coeffs_stride);
+  return ntt_lde(io, l, B, ti, tf, st, coeffs, coeffs_stride, plan_only);
 }
 
 // ------------------------------------------------------------------ bit reversal
@@ -1979,7 +1985,8 @@ int vs_ntt_plan_candidates(uint32_t log_n, uint32_t* out, uint32_t cap, uint32_t
 
 // Times every candidate plan of log_n on an n_cols-column LDE (stwo convention,
 // seeded columns, `reps` timed runs after one warm-up each, CUDA events on the
-// stream) and keeps the fastest as the plan of log_n.
+// stream) and keeps the fastest as the plan of log_n. A job that small is timed in its
+// plans' passes all the same: the plan serves the size's larger jobs.
 int vs_autotune_lde(uint32_t log_n, uint32_t n_cols, uint32_t blowup_bits, uint32_t reps, uint32_t* best,
                     float* ms_out, uint32_t cap, vs_stream_t stream) {
   clear_error();
@@ -2005,10 +2012,10 @@ int vs_autotune_lde(uint32_t log_n, uint32_t n_cols, uint32_t blowup_bits, uint3
   NttPlan best_plan = saved;
   for (size_t i = 0; i < cands.size() && rc == VS_OK; i++) {
     set_plan(log_n, cands[i]);
-    rc = lde_cached(TW_STWO, src, n, dst, N, n_cols, log_n, blowup_bits, st);
+    rc = lde_cached(TW_STWO, src, n, dst, N, n_cols, log_n, blowup_bits, st, nullptr, 0, true);
     if (rc == VS_OK) rc = check_cuda(cudaEventRecord(e0, st), "vs_autotune_lde event");
     for (uint32_t k = 0; k < reps && rc == VS_OK; k++)
-      rc = lde_cached(TW_STWO, src, n, dst, N, n_cols, log_n, blowup_bits, st);
+      rc = lde_cached(TW_STWO, src, n, dst, N, n_cols, log_n, blowup_bits, st, nullptr, 0, true);
     if (rc == VS_OK) rc = check_cuda(cudaEventRecord(e1, st), "vs_autotune_lde event");
     if (rc == VS_OK) rc = check_cuda(cudaEventSynchronize(e1), "vs_autotune_lde sync");
     float ms = 0.f;

@@ -65,11 +65,12 @@ int tw_for(int kind, uint32_t log_n, bool forward, NttTw* out, cudaStream_t st);
 // Full transform (in place when src == dst).
 int ntt_transform(const NttColumns& io, uint32_t log_n, const NttTw& tw, bool forward, cudaStream_t st);
 // interpolate(log_n) -> zero-pad -> evaluate(log_n + B); src is left untouched. With
-// coeffs, column c's coefficients also go to coeffs + c * coeffs_stride.
+// coeffs, column c's coefficients also go to coeffs + c * coeffs_stride. plan_only: not in
+// the small-job passes (the autotuner times plans).
 int ntt_lde(const NttColumns& io, uint32_t log_n, uint32_t B, const NttTw& tw_inv, const NttTw& tw_fwd,
-            cudaStream_t st, uint32_t* coeffs = nullptr, uint64_t coeffs_stride = 0);
+            cudaStream_t st, uint32_t* coeffs = nullptr, uint64_t coeffs_stride = 0, bool plan_only = false);
 int lde_cached(int kind, const uint32_t* src, uint64_t src_stride, uint32_t* dst, uint64_t dst_stride,
                uint32_t n_cols, uint32_t log_n, uint32_t B, cudaStream_t st, uint32_t* coeffs = nullptr,
-               uint64_t coeffs_stride = 0);
+               uint64_t coeffs_stride = 0, bool plan_only = false);
 
 }  // namespace vs
