@@ -40,6 +40,13 @@
 #include "vs_common.cuh"
 #include "vs_field.cuh"
 
+// Every launch in clusters goes through this function, which is no inline one so that a test
+// can load one that refuses in its place.
+extern "C" __attribute__((noinline)) int vs_internal_cluster_launch(const cudaLaunchConfig_t* cfg, const void* fn,
+                                                                    void** args) {
+  return (int)cudaLaunchKernelExC(cfg, fn, args);
+}
+
 namespace vs {
 
 // Shared-tile swizzle: the 16-byte chunk index (word bits 2..4) is XORed with
@@ -1523,6 +1530,28 @@ bool strided_aligned(const NttColumns& io) {
 }
 }  // namespace
 
+// A launch of fn(args...) in clusters; *launched says whether the runtime took it (it may
+// not, for instance under an MPS partition too small to co-schedule a cluster).
+template <class... Args>
+static void launch_clusters(const void* fn, dim3 grid, uint32_t threads, uint32_t smem, dim3 cluster, bool* launched,
+                           cudaStream_t st, Args... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = threads;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = cluster.x;
+  attr[0].val.clusterDim.y = cluster.y;
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  void* argv[] = {&args...};
+  *launched = vs_internal_cluster_launch(&cfg, fn, argv) == cudaSuccess;
+  if (!*launched) cudaGetLastError();  // the refused launch's error
+}
+
 static int ntt_transform_aligned(const NttColumns& io, uint32_t L, const NttTw& tw, bool fwd, cudaStream_t st);
 
 int ntt_transform(const NttColumns& io, uint32_t L, const NttTw& tw, bool fwd, cudaStream_t st) {
@@ -1663,56 +1692,37 @@ static int ntt_lde_aligned(const NttColumns& io, uint32_t l, uint32_t B, const N
     pf.dst_stride = io.dst_stride;
     pi.dst = coeffs;
     pi.dst_stride = coeffs_stride;
-    const uint32_t M = r.b - r.a + 1, T = M + r.c;
-    if (small) {
-      cudaLaunchConfig_t cfg = {};
-      cfg.gridDim = dim3(io.n_cols << (l - T), 1u << B);
-      cfg.blockDim = 1u << (T - 3);
-      cfg.dynamicSmemBytes = (9u << T) / 8 * 4;
-      cfg.stream = st;
-      cudaLaunchAttribute attr[1];
-      attr[0].id = cudaLaunchAttributeClusterDimension;
-      attr[0].val.clusterDim.x = 1;
-      attr[0].val.clusterDim.y = 1u << B;
-      attr[0].val.clusterDim.z = 1;
-      cfg.attrs = attr;
-      cfg.numAttrs = 1;
-      VS_CUDA(cudaLaunchKernelEx(&cfg, small_top_fn(M, r.c), pi, pf, io.n_cols));
-      VS_LAUNCHED("ntt_lde_top_small_kernel");
-    } else {
-      TopFn fn = top_fn(M, r.c, plan.radix);
-      if (!fn) return set_error(VS_ERR_INVALID, "ntt: no LDE kernel for shape M=%u C=%u", M, r.c);
+    const uint32_t M = r.b - r.a + 1;
+    bool launched = false;
+    if (small) {  // a tile's blocks as one cluster
+      const uint32_t T = M + r.c;
+      launch_clusters((const void*)small_top_fn(M, r.c), dim3(io.n_cols << (l - T), 1u << B), 1u << (T - 3),
+                      (9u << T) / 8 * 4, dim3(1, 1u << B), &launched, st, pi, pf, io.n_cols);
+    }
+    if (!launched) {
+      // where the cluster is refused, a small job's top pass runs on 8192-word tiles
+      if (small && r.c) pi.c = pf.c = kMaxT - M;
+      const uint32_t C = pf.c, T = M + C;
+      if (small && !C && coeffs)  // which leave no coefficients up to 13 layers
+        VS_TRY(ntt_transform({io.src, coeffs, nullptr, nullptr, io.src_stride, coeffs_stride, io.n_cols}, l, tw_inv, false, st));
+      TopFn fn = top_fn(M, C, small ? 3 : plan.radix);
+      if (!fn) return set_error(VS_ERR_INVALID, "ntt: no LDE kernel for shape M=%u C=%u", M, C);
       const uint32_t smem = 8u << T;  // working tile + coefficient tile
-      const dim3 grid(1u << (l - T), io.n_cols), block(1u << (T - 5));
-      // 16-byte-row tiles run as CTA pairs (whole-sector tile stores); if the
-      // cluster launch is refused, the plain kernel runs instead
-      TopFn cfn = nullptr;
-      const uint32_t K = kTopPair;
-      if (plan.radix != 5 && M == 11 && r.c == 2) cfn = top_hi_pair();
-      bool launched = false;
-      if (cfn && grid.x % K == 0) {
-        VS_TRY(allow_smem((const void*)cfn, smem));
-        cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = grid;
-        cfg.blockDim = block;
-        cfg.dynamicSmemBytes = smem;
-        cfg.stream = st;
-        cudaLaunchAttribute attr[1];
-        attr[0].id = cudaLaunchAttributeClusterDimension;
-        attr[0].val.clusterDim.x = K;
-        attr[0].val.clusterDim.y = 1;
-        attr[0].val.clusterDim.z = 1;
-        cfg.attrs = attr;
-        cfg.numAttrs = 1;
-        if (cudaLaunchKernelEx(&cfg, cfn, pi, pf, B) == cudaSuccess) launched = true;
-        else cudaGetLastError();  // clear the refused launch's error
+      const dim3 grid(1u << (l - T), io.n_cols);
+      const uint32_t threads = 1u << (T - 5), K = kTopPair;
+      // 16-byte-row tiles run as CTA pairs (whole-sector tile stores); where those are
+      // refused, as single CTAs
+      if (plan.radix != 5 && M == 11 && C == 2 && grid.x % K == 0) {
+        TopFn pair = top_hi_pair();
+        VS_TRY(allow_smem((const void*)pair, smem));
+        launch_clusters((const void*)pair, grid, threads, smem, dim3(K), &launched, st, pi, pf, B);
       }
       if (!launched) {
         VS_TRY(allow_smem((const void*)fn, smem));
-        fn<<<grid, block, smem, st>>>(pi, pf, B);
+        fn<<<grid, threads, smem, st>>>(pi, pf, B);
       }
-      VS_LAUNCHED("ntt_lde_top_kernel");
     }
+    VS_LAUNCHED("LDE top pass");
   }
   // 3. forward passes below the top one over the whole evaluation domain
   for (int i = (int)np - 2; i >= 0; i--) {
