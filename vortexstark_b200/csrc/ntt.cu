@@ -1265,8 +1265,8 @@ static const uint32_t kMinC = 2;   // >= 16-byte contiguous runs per tile row
 //  * LDEs above: 2 x 2^14 x4 24.9 -> 17.1, 4 x 2^16 x4 (2^20) 27.0 -> 22.9, 2 x 2^18 x2
 //    (2^20) 25.7 -> 23.0, but 7 x 2^17 x2 (1.75 x 2^20) 29.1 -> 29.2 and 34 x 2^14 x2
 //    (1.06 x 2^20) 23.0 -> 25.0: the repeated inverse layers then cost more than the
-//    idle SMs they fill. LDEs without a blowup repeat none, but 48 x 2^14 (3 x 2^18) takes
-//    21.6 -> 22.8, 34 x 2^14 21.5 -> 18.5.
+//    idle SMs they fill. Without a blowup none is repeated (2 x 2^19 24.7 -> 22.6), but
+//    2^14 rows stop gaining earlier (34 x 2^14 21.5 -> 18.5, 48 x 2^14 21.6 -> 22.8).
 // Most evaluation words of an LDE for that. Up to 13 layers the word rounds run a column's
 // blocks one after the other in one CTA, so many columns fill the chip and leave nothing to
 // gain: from ten layers on the line lies at one wave of 1024-thread CTAs up to x2 (148 x
@@ -1277,7 +1277,7 @@ static const uint32_t kMinC = 2;   // >= 16-byte contiguous runs per tile row
 // stop at 32 an SM (1024 x 2^5 x4 10.3 either way, 4096 columns 24.7 -> 30.8).
 static uint64_t small_lde_words(uint32_t l, uint32_t B) {
   constexpr uint64_t wave = 148ull << 13;
-  if (l > 13) return B ? 1ull << 20 : 5ull << 17;
+  if (l > 13) return l == 14 && !B ? 5ull << 17 : 1ull << 20;
   if (l == 5 && B > 1) return wave >> 3;
   if (l < 10 || (B == 0 && l < 13)) return B == 3 ? 3ull << 20 : 1ull << 22;
   return B == 3 ? 2 * wave : B == 2 ? 3ull << 19 : wave;
