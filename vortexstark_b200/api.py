@@ -13,9 +13,6 @@ import torch
 
 from . import check, lib
 
-PROOF_CAP = 32 << 20  # bytes; more than the largest proof (log_n = 28: a few MB)
-
-
 
 def _stream(stream=None) -> int:
     s = stream if stream is not None else torch.cuda.current_stream()

@@ -13,9 +13,12 @@
 //     concatenation of the jobs' levels (parents never straddle jobs either);
 //   * fused quotient / fold leaves: the leaf functors split a global leaf index
 //     into (job, index) and read the job's own challenges;
-//   * Fiat-Shamir channel: one thread per job (one CTA per job for the query
-//     draw, whose squeezes are independent given the state);
-//   * decommitment: one warp per (job, query) gathers its authentication path.
+//   * Fiat-Shamir channel: the launch that ends a tree mixes its root and draws the
+//     next challenge, one thread a job (transcript_tree.cuh);
+//   * the FRI layers of 2^9 values and fewer, and the query draw (whose squeezes are
+//     independent given the state): one launch, a CTA a job;
+//   * decommitment: one launch over all trees, one warp per (job, query) gathers its
+//     authentication path.
 //
 // Trees keep every level from level 3 up (eight-leaf groups; 6 in the trees of single
 // proofs above 2^22 leaves): an authentication path is a gather of the stored
@@ -49,7 +52,7 @@ namespace {
 constexpr int BMAXF = 28;  // FRI layers for log_eval <= 30
 // Lowest kept level of a tree of 2^m leaves: an opened leaf's group of 2^s is hashed again.
 // Eight-leaf groups cost 8 bytes a leaf; trees above 2^22 leaves keep 64-leaf groups (1
-// byte a leaf), which one warp still hashes at once.
+// byte a leaf), which one warp hashes in two steps.
 constexpr uint32_t BGROUP_MAX = 6;
 constexpr uint32_t group_log(uint32_t m) { return m > 22 ? BGROUP_MAX : (m < 3 ? m : 3); }
 

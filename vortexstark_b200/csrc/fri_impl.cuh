@@ -25,15 +25,13 @@ struct Soa4Out {
 };
 
 // Folded SoA4 layer as Merkle leaves: leaf i = fold(src[2i], src[2i+1]); written to dst.
-// circle = true also accumulates dst = dst * alpha^2 + f' when accumulate is set
-// (fri.cu:44-78); the prover's destination starts at zero, so accumulate = false
-// there and dst is not read.
+// (The circle fold's accumulation dst * alpha^2 + f', fri.cu:44-78, has nothing to add
+// in a prover, whose destination starts at zero.)
 struct LeafFold {
   Soa4Ptrs src;
   Soa4Out dst;
   const uint32_t* tw;
-  qm31 alpha, alpha_sq;
-  int accumulate;
+  qm31 alpha;
   __device__ __forceinline__ void operator()(uint64_t i, uint32_t out[8]) const {
     uint2 a0 = ld2(src.c[0] + 2 * i);
     uint2 a1 = ld2(src.c[1] + 2 * i);
@@ -41,10 +39,6 @@ struct LeafFold {
     uint2 a3 = ld2(src.c[3] + 2 * i);
     qm31 f0{{a0.x, a1.x, a2.x, a3.x}}, f1{{a0.y, a1.y, a2.y, a3.y}};
     qm31 r = fold_pair(f0, f1, alpha, __ldg(tw + i));
-    if (accumulate) {
-      qm31 prev{{dst.c[0][i], dst.c[1][i], dst.c[2][i], dst.c[3][i]}};
-      r = qadd(qmul(prev, alpha_sq), r);
-    }
 #pragma unroll
     for (int k = 0; k < 4; k++) dst.c[k][i] = r.v[k];
     uint32_t m[16] = {0};
@@ -56,14 +50,14 @@ struct LeafFold {
   }
 };
 
-// The same leaf without accumulation, its challenge (4 words) in device memory.
+// The same leaf, its challenge (4 words) in device memory.
 struct LeafFoldAt {
   Soa4Ptrs src;
   Soa4Out dst;
   const uint32_t* tw;
   const uint32_t* alpha;
   __device__ __forceinline__ void operator()(uint64_t i, uint32_t out[8]) const {
-    LeafFold f{src, dst, tw, qm31{{__ldg(alpha), __ldg(alpha + 1), __ldg(alpha + 2), __ldg(alpha + 3)}}, qzero(), 0};
+    LeafFold f{src, dst, tw, qm31{{__ldg(alpha), __ldg(alpha + 1), __ldg(alpha + 2), __ldg(alpha + 3)}}};
     f(i, out);
   }
 };

@@ -97,17 +97,18 @@ __global__ void __launch_bounds__(MK_THREADS) channel_tile_kernel(Leaf leaf, Tre
   if (k + TL == t.m && threadIdx.x == 0) channel_step(step, blockIdx.x, root, root + 8);
 }
 
-// The last FRI layers (2^TAIL_LOG values and fewer), one CTA per job: folds from shared memory, trees and challenges without
-// leaving the SM. As separate launches each of these layers took about 12 us.
+// The last FRI layers (2^TAIL_LOG values and fewer), one CTA per job: folds from shared
+// memory, trees and challenges without leaving the SM. As separate launches each of these
+// layers took about 12 us.
 // Layer l has 2^(log_eval-1-l) values; its challenge is at alpha0 + 4 l of the job's slots.
 constexpr uint32_t TAIL_LOG = 9;
 constexpr int TAIL_MAXF = 28;
 constexpr uint32_t TAIL_TILE_WORDS = 12u << TAIL_LOG;  // merkle_smem_bytes(TAIL_LOG) / 4
 struct FriTail {
-  uint32_t first, nf, log_eval;        // layers first (>= 1) .. nf - 1
+  uint32_t first, nf, log_eval;        // layers first .. nf - 1
   uint32_t alpha0;
   const uint32_t* tw[TAIL_MAXF];
-  const uint32_t* in[4];               // layer first - 1: planes [jobs][2^(log_eval-first)]
+  const uint32_t* in[4];               // what layer first folds: planes [jobs][2^(log_eval-first)]
   uint32_t* fri[TAIL_MAXF][4];         // planes [jobs][2^(log_eval-1-l)]
   TreeLevels tree[TAIL_MAXF];
   ChannelStep step;                    // of layer first
