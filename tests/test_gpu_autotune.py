@@ -116,21 +116,22 @@ def default_split():
         api.set_merkle_split(0)
 
 
-@pytest.mark.parametrize("log_n,n_cols", [(11, 34), (15, 34), (17, 5)])
-def test_every_split_gives_the_oracle_roots(L, default_split, log_n, n_cols):
-    from gpu_util import u32_host
+@pytest.mark.parametrize("log_n,n_cols,fri_log", [(15, 34, 15), (20, 18, 12), (21, 2, 22)])
+def test_every_split_gives_the_oracle_roots(L, default_split, log_n, n_cols, fri_log):
+    """The split shapes trees of 2^20 leaves and more and, up to 5, the large FRI layers (two of the
+    chain of 2^22 values); smaller ones take no notice of it."""
     rng = np.random.default_rng(900 + log_n)
     cols = rand_m31(rng, n_cols, 1 << log_n)
-    exp_rp = O.merkle_root_rowpacked(cols, threads=4)
+    exp_rp = O.merkle_root_rowpacked(cols, threads=8)
     n_cap = min(16, n_cols)
-    exp_cap = O.merkle_root_capped(cols[:n_cap], threads=4)
-    fri_log = log_n
+    exp_cap = O.merkle_root_capped(cols[:n_cap], threads=8)
     src = rand_m31(rng, 4, 1 << fri_log)
     alphas = rand_m31(rng, fri_log - 3, 4)
     er = np.zeros((fri_log - 3, 8), np.uint32)
     el = np.zeros((8, 4), np.uint32)
-    O.lib().oracle_bench_fri(O.ptr_array(list(src)), fri_log, O.ptr(alphas.reshape(-1).copy()), 4, O.ptr(er), O.ptr(el))
-    d_cols = dev(cols.reshape(-1))
+    O.lib().oracle_bench_fri(O.ptr_array(list(src)), fri_log, O.ptr(alphas.reshape(-1).copy()), 8, O.ptr(er), O.ptr(el))
+    d_cols, d_src = dev(cols.reshape(-1)), dev(src.reshape(-1))
+    work, roots, last = empty(4 << fri_log), empty(8 * (fri_log - 3)), empty(32)
     for split in range(9):
         api.set_merkle_split(split)
         root = empty(8)
@@ -138,15 +139,14 @@ def test_every_split_gives_the_oracle_roots(L, default_split, log_n, n_cols):
         assert np.array_equal(host(root), exp_rp), split
         V.check(L.vs_merkle_root_capped(ptr(d_cols), 1 << log_n, n_cap, log_n, ptr(root), None), "capped")
         assert np.array_equal(host(root), exp_cap), split
-        work, roots, last = empty(4 << fri_log), empty(8 * (fri_log - 3)), empty(32)
-        V.check(L.vs_fri_fold_commit(ptr(dev(src.reshape(-1))), fri_log, u32_host(alphas.reshape(-1)), ptr(work),
+        V.check(L.vs_fri_fold_commit(ptr(d_src), fri_log, u32_host(alphas.reshape(-1)), ptr(work),
                                      ptr(roots), ptr(last), None), "vs_fri_fold_commit")
         assert np.array_equal(host(roots).reshape(-1, 8), er), split
         assert np.array_equal(host(last).reshape(8, 4), el), split
 
 
 def test_autotune_merkle_keeps_a_split(L, default_split):
-    res = api.autotune_merkle(16, n_cols=34, reps=2)
+    res = api.autotune_merkle(21, n_cols=34, reps=2)
     assert 0 <= res["best"] <= 8 and api.merkle_split() == res["best"]
     assert all(t > 0 for t in res["ms"]) and res["ms"][res["best"]] == min(res["ms"])
 
@@ -170,8 +170,9 @@ def test_autotune_merkle_reports_the_split_that_runs(L, default_split):
 
 @pytest.mark.parametrize("split", [1, 5, 8])
 def test_prover_trees_with_split_match_oracle(L, default_split, split):
-    """Proof trees of 2^20 leaves (log_n 18) go through 2^min(split, 5) subtree
-    roots per tile in both provers; the bytes stay the oracle's."""
+    """The graph prover's trees of 2^20 leaves (log_n 18) go through 2^min(split, 5) subtree
+    roots per tile; the bytes stay the oracle's, as do those of vs_prove_fib, whose trees
+    keep their lower levels and take no notice of the split."""
     import ctypes as C
     exp = O.prove(3, 77, 18)
     api.set_merkle_split(split)

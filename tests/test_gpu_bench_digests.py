@@ -3,7 +3,7 @@ oracle's results (tests/golden/bench_digests.json, written by
 tests/golden/gen_bench_digests.py, which runs the oracle for minutes).
 
 * the commitment-layer step of bench.py: 34 columns x 2^24 rows, x4 stwo LDE,
-  row-packed root (at split 0 and the largest split), and the FRI fold+commit of
+  row-packed root (at the default and the largest split), and the FRI fold+commit of
   the seeded 2^26 QM31 vector: 23 layer roots and the last layer;
 * the 64-job batched mix (log_n 16..22 Fibonacci proofs and 1..34-column
   commitments) through the batching engine and through the plain path;

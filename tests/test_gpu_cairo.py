@@ -316,10 +316,10 @@ def test_tile_tree_paths_rejects_bad_arguments(L):
     assert L.vs_tile_tree_paths(7, hc, 4, 6, ptr(t), ix, 0, out, out, None) != 0   # unknown leaf
 
 
-@pytest.mark.parametrize("split", [0, 5])
+@pytest.mark.parametrize("split", [0, 1, 5, 8])
 def test_group_commit_tile_roots_with_split(L, split):
     """2^20 evaluation rows: the tile roots go through 2^split subtree roots per tile
-    when a split is set; roots and tile roots stay the oracle's."""
+    (2^7 when none is set); roots and tile roots stay the oracle's."""
     from vortexstark_b200 import api
     log_n, nc = 18, 2
     n = 1 << log_n

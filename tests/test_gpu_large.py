@@ -37,8 +37,9 @@ def test_full_size_proof_matches_oracle_digest(key):
 @pytest.mark.parametrize("split", [3, 5])
 @pytest.mark.parametrize("key", sorted(CASES, key=lambda k: [int(x) for x in k.split(":")]))
 def test_full_size_proof_with_merkle_split(key, split):
-    """The prover's trees of 2^20+ leaves reach their tile roots through 2^split
-    subtree roots per tile; the proof bytes must not change."""
+    """The graph prover's trees of 2^20+ leaves reach their tile roots through 2^split
+    subtree roots per tile; the proof bytes must not change, and vs_prove_fib's (which has
+    no such trees) are the same."""
     if not torch.cuda.is_available():
         pytest.skip("no CUDA device")
     c = CASES[key]

@@ -49,8 +49,8 @@ def _oracle_root(n_cols, log_n, seed):
 
 
 def test_noalloc_matches_allocating_root_twice(L):
-    first = _cols(34, 16, 0x1001)   # uses the scratch array (64 subtree roots)
-    second = _cols(5, 21, 0x1002)   # reuses it with different contents (2048 + 2 roots)
+    first = _cols(34, 16, 0x1001)   # uses the scratch array (128 subtree roots)
+    second = _cols(5, 21, 0x1002)   # reuses it with different contents (2^16 + 2^7 roots)
     for cols, log_n, seed in ((first, 16, 0x1001), (second, 21, 0x1002)):
         a, b = _roots(L, cols, log_n)
         assert np.array_equal(a, b)
