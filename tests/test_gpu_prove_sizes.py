@@ -9,12 +9,23 @@ pytestmark = pytest.mark.gpu
 
 torch = pytest.importorskip("torch")
 import oracle_lib as O  # noqa: E402
+from gpu_util import small_pool  # noqa: E402
 from vortexstark_b200 import api  # noqa: E402
 
 
 @pytest.mark.parametrize("log_n", [4, 7, 9, 13, 15, 17, 18])
 def test_proof_bytes(log_n):
     assert api.prove_fib(3, 1000 + log_n, log_n) == O.prove(3, 1000 + log_n, log_n)
+
+
+@pytest.mark.parametrize("log_n", [16, 18])
+def test_proof_where_the_workspace_cannot_be_allocated(log_n):
+    """180 bytes a row do not fit beside what is held, 96 do: trees keep fewer levels."""
+    exp = O.prove(5, 50 + log_n, log_n)
+    assert api.prove_fib(5, 50 + log_n, log_n) == exp  # tables of the size are cached from here on
+    with small_pool(64 << 20) as pool:
+        pool.hold((64 << 20) - (130 << log_n))
+        assert api.prove_fib(5, 50 + log_n, log_n) == exp
 
 
 def test_threads_and_streams():

@@ -55,6 +55,8 @@ constexpr int BMAXF = 28;  // FRI layers for log_eval <= 30
 // byte a leaf), which one warp hashes in two steps.
 constexpr uint32_t BGROUP_MAX = 6;
 constexpr uint32_t group_log(uint32_t m) { return m > 22 ? BGROUP_MAX : (m < 3 ? m : 3); }
+// 64-leaf groups in every tree, where the device has no room for more levels.
+constexpr uint32_t group_most(uint32_t m) { return std::min(m, BGROUP_MAX); }
 
 // ------------------------------------------------------------------ batched leaf functors
 // Global leaf g of a batch of trees with 2^log_len leaves each: job g >> log_len,
@@ -224,6 +226,7 @@ uint64_t align256(uint64_t b) { return (b + 255) & ~255ull; }
 struct BatchProver::Impl {
   uint32_t log_n = 0, log_eval = 0, nf = 0, cap = 0, astride = 0;
   uint64_t n = 0, N = 0, total = 0;
+  uint32_t (*group)(uint32_t) = group_log;
   int device = 0;
   cudaStream_t st = nullptr, running = nullptr;
   uint32_t count = 0;  // jobs of the batch in flight
@@ -268,7 +271,7 @@ struct BatchProver::Impl {
       for (int k = 0; k < 4; k++) fri[l][k] = (uint32_t*)take(4 * half * cap);
     }
     auto tree = [&](TreeLevels& t, uint32_t m) {
-      t = TreeLevels{nullptr, cap, group_log(m), m};
+      t = TreeLevels{nullptr, cap, group(m), m};
       t.base = (uint32_t*)take(TreeLevels::bytes(cap, t.s, m));
     };
     tree(trace_t, log_eval);
@@ -428,6 +431,12 @@ int BatchProver::prove_once(uint32_t a, uint32_t b, uint32_t log_n, uint8_t* out
                      (unsigned long long)cap);
   uint8_t* mem = nullptr;
   cudaError_t e = cudaMallocAsync((void**)&mem, p.total, st);
+  if (e == cudaErrorMemoryAllocation) {  // 96 bytes a row instead of 180, for traces up to 2^20 rows
+    cudaGetLastError();
+    p.group = group_most;
+    p.plan(log_n, 1);
+    e = cudaMallocAsync((void**)&mem, p.total, st);
+  }
   if (e != cudaSuccess)
     return set_error(VS_ERR_OOM, "proof workspace (%llu bytes): %s", (unsigned long long)p.total, cudaGetErrorString(e));
   p.carve(mem);
