@@ -9,7 +9,8 @@ pytestmark = pytest.mark.gpu
 
 torch = pytest.importorskip("torch")
 import oracle_lib as O  # noqa: E402
-from gpu_util import small_pool  # noqa: E402
+from gpu_util import ptr, small_pool, zeros  # noqa: E402
+import vortexstark_b200 as V  # noqa: E402
 from vortexstark_b200 import api  # noqa: E402
 
 
@@ -26,6 +27,15 @@ def test_proof_where_the_workspace_cannot_be_allocated(log_n):
     with small_pool(64 << 20) as pool:
         pool.hold((64 << 20) - (130 << log_n))
         assert api.prove_fib(5, 50 + log_n, log_n) == exp
+
+
+def test_a_refused_workspace_does_not_fail_the_next_call():
+    cols, root = zeros(3 << 8), zeros(8)
+    with small_pool(32 << 20) as pool:
+        pool.hold(32 << 20)
+        with pytest.raises(V.VstarkError):
+            api.prove_fib(1, 2, 12)
+        V.check(V.lib().vs_merkle_root_rowpacked(ptr(cols), 1 << 8, 3, 8, ptr(root), None), "no scratch needed")
 
 
 def test_threads_and_streams():

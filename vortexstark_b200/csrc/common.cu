@@ -19,6 +19,9 @@ int set_error(int status, const char* fmt, ...) {
   va_start(ap, fmt);
   vsnprintf(g_err, sizeof g_err, fmt, ap);
   va_end(ap);
+  // A refused allocation or launch is reported by this call: the next one's launch check
+  // must not find it again.
+  if (status == VS_ERR_CUDA || status == VS_ERR_OOM) cudaGetLastError();
   return status;
 }
 void clear_error() { g_err[0] = 0; }
