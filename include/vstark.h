@@ -330,8 +330,8 @@ int vs_fri_fold_commit(const uint32_t* d_src, uint32_t log_n, const uint32_t* h_
  * wire format (src/bin/stark_cli.rs:907-976) into h_out (host) when cap is large
  * enough; *out_len receives the proof length. With h_out NULL or too small a cap
  * nothing is proved: VS_ERR_INVALID, and the length. Takes one stream-ordered workspace for
- * the call, about 180 bytes a row up to 2^20 rows (96 where that cannot be allocated) and 96
- * above. */
+ * the call, about 180 bytes a row up to 2^20 rows and 100 to 125 above, or 96 where that
+ * cannot be allocated. */
 int vs_prove_fib(uint32_t a, uint32_t b, uint32_t log_n, uint8_t* h_out, uint64_t cap, uint64_t* out_len,
                  vs_stream_t stream);
 /* Verifier (src/verifier.rs:39-236) over a KRAK proof. Returns VS_OK when

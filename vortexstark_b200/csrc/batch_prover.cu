@@ -431,7 +431,7 @@ int BatchProver::prove_once(uint32_t a, uint32_t b, uint32_t log_n, uint8_t* out
                      (unsigned long long)cap);
   uint8_t* mem = nullptr;
   cudaError_t e = cudaMallocAsync((void**)&mem, p.total, st);
-  if (e == cudaErrorMemoryAllocation) {  // 96 bytes a row instead of 180, for traces up to 2^20 rows
+  if (e == cudaErrorMemoryAllocation) {  // 96 bytes a row instead of 100 to 180
     cudaGetLastError();
     p.group = group_most;
     p.plan(log_n, 1);
