@@ -1167,7 +1167,7 @@ template <int M> TopFn top5_hi() { return ntt_lde_top_kernel<M, 13 - M>; }
 constexpr uint32_t kSmallMaxL = 19, kSmallUpperC = 3;
 using SmallFn = void (*)(NttPass, uint32_t);
 using SmallTopFn = void (*)(NttPass, NttPass, uint32_t);
-#define VS_SMALL_LO VS_SM(5, 0) VS_SM(6, 0) VS_SM(7, 0) VS_SM(8, 0) VS_SM(9, 0) VS_SM(10, 0) VS_SM(11, 0) VS_SM(12, 0) VS_SM(13, 0)
+#define VS_SMALL_LO VS_SM(5, 0) VS_SM(6, 0) VS_SM(7, 0) VS_SM(8, 0) VS_SM(9, 0) VS_SM(10, 0) VS_SM(11, 0) VS_SM(12, 0)
 #define VS_SMALL_HI VS_SM(7, 3) VS_SM(8, 3) VS_SM(9, 3)
 static SmallFn small_fn(bool fwd, uint32_t M, uint32_t C) {
   switch (16 * M + C) {
@@ -1180,7 +1180,7 @@ static SmallFn small_fn(bool fwd, uint32_t M, uint32_t C) {
 static SmallTopFn small_top_fn(uint32_t M, uint32_t C) {
   switch (16 * M + C) {
 #define VS_SM(m, c) case 16 * m + c: return ntt_lde_top_small_kernel<m, c>;
-    VS_SMALL_LO VS_SMALL_HI
+    VS_SMALL_LO VS_SM(13, 0) VS_SMALL_HI
 #undef VS_SM
     default: return nullptr;
   }
@@ -1260,7 +1260,8 @@ static const uint32_t kMaxT = 13;  // tile of 8192 words (32 KiB), 256 threads
 static const uint32_t kMinC = 2;   // >= 16-byte contiguous runs per tile row
 // Jobs of few words (all columns together) run in the small-job passes, whatever the plan of
 // their size: that was tuned on, or set for, jobs that fill the chip. Measured (us, 8192-word tiles then small-job passes):
-//  * transforms: 2^14 21.6 -> 17.1, 2^19 23.9 -> 20.5, but 2^20 23.9 -> 25.7;
+//  * transforms: 2^14 21.6 -> 17.1, 2^19 23.9 -> 20.5, but 2^20 23.9 -> 25.7, and 2^13, one
+//    pass of one tile either way, 16.7 -> 17.7;
 //  * LDEs of at most 13 layers: 34 x 2^10 x4 14.4 -> 5.8, 34 x 2^13 x8 43.0 -> 32.9;
 //  * LDEs above: 2 x 2^14 x4 24.9 -> 17.1, 4 x 2^16 x4 (2^20) 27.0 -> 22.9, 2 x 2^18 x2
 //    (2^20) 25.7 -> 23.0, but 7 x 2^17 x2 (1.75 x 2^20) 29.1 -> 29.2 and 34 x 2^14 x2
@@ -1287,7 +1288,7 @@ static bool default_plan(uint32_t L) {
   return p.lower == 0 && p.items == 0 && p.radix == 3;
 }
 static bool small_transform_job(uint32_t L, uint64_t words) {
-  return L >= 5 && L <= kSmallMaxL && words <= (1ull << 19);
+  return L >= 5 && L <= kSmallMaxL && L != 13 && words <= (1ull << 19);
 }
 static bool small_lde_job(uint32_t l, uint32_t B, uint32_t n_cols) {
   uint64_t most = small_lde_words(l, B);
