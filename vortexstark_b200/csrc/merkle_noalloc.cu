@@ -23,8 +23,8 @@ constexpr uint32_t NOALLOC_MAX_LOG_LEAVES = 26;
 constexpr uint64_t NOALLOC_SCRATCH_WORDS = ((1ull << (NOALLOC_MAX_LOG_LEAVES - 10)) + 128) * 8;  // 2.1 MB
 
 // Every GPU that loads the library holds this array until the process exits.
-// All calls above 1024 leaves share it on a device and it keeps the last call's contents; calls
-// whose work overlaps on the GPU would race on it.
+// All calls above 1024 leaves share it on a device and it keeps the last call's contents;
+// such calls whose work overlaps on the GPU would race on it.
 static __device__ __align__(256) uint32_t g_noalloc_scratch[NOALLOC_SCRATCH_WORDS];
 
 namespace {

@@ -1259,7 +1259,8 @@ __global__ void scale_kernel(uint32_t* __restrict__ d, uint32_t s, uint32_t n) {
 static const uint32_t kMaxT = 13;  // tile of 8192 words (32 KiB), 256 threads
 static const uint32_t kMinC = 2;   // >= 16-byte contiguous runs per tile row
 // Jobs of few words (all columns together) run in the small-job passes, whatever the plan of
-// their size: that was tuned on, or set for, jobs that fill the chip. Measured (us, 8192-word tiles then small-job passes):
+// their size: that was tuned on, or set for, jobs that fill the chip. Measured (us,
+// 8192-word tiles or word rounds, then small-job passes):
 //  * transforms: 2^14 21.6 -> 17.1, 2^19 23.9 -> 20.5, but 2^20 23.9 -> 25.7, and 2^13, one
 //    pass of one tile either way, 16.7 -> 17.7;
 //  * LDEs of at most 13 layers: 34 x 2^10 x4 14.4 -> 5.8, 34 x 2^13 x8 43.0 -> 32.9;
